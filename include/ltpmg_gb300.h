@@ -110,6 +110,8 @@ typedef struct {
      *                8 insert, 9 finish
      * priority rule: 0 mark, 1 ids, 2 min-writer, 3 abort, 4 execute,
      *                8 insert, 9 finish
+     * ordered rule, batches of up to 2^21 ops that are executed by buckets of
+     * cells: 0 split, 7 buckets, 8 insert, 9 finish
      * and 11 the whole batch */
     float ms_stage[LTP_N_STAGES];
 } ltp_stats;

@@ -20,7 +20,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompil
               "-I", os.path.join(ROOT, "include")]
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-Wall", "-I", os.path.join(ROOT, "include")]
 
-CU_SOURCES = ["ltp_kernels.cu", "ltp_api.cu", "ltp_noalloc.cu", "ltp_ingest.cu"]
+CU_SOURCES = ["ltp_kernels.cu", "ltp_buckets.cu", "ltp_api.cu", "ltp_noalloc.cu", "ltp_ingest.cu"]
 # the benchmark's random-access probe: its own library, outside the product
 PROBE_SOURCE = "ltp_probe.cu"
 PROBE_LIB = os.path.join(PKG, "libltpmg_probe.so")

@@ -82,8 +82,10 @@ void free_scratch_ops(Scratch &s) {
 void free_scratch_words(Scratch &s) {
     cudaFree(s.words);
     cudaFree(s.cview);
+    cudaFree(s.word_epoch);
     s.words = nullptr;
     s.cview = nullptr;
+    s.word_epoch = nullptr;
 }
 
 // Sizes the bitmaps to the cell space and the per-op scratch to n_ops.
@@ -98,6 +100,11 @@ int ensure_scratch(ltp_ctx *ctx, uint64_t n_ops) {
         CK(cudaMemset(s.words, 0, (words + 1) * sizeof(WordState)));
         CK(dalloc(&s.cview, words + 1));  // 8 B per 32 cells; the 64-cell view takes 16 B per word
         CK(cudaMemset(s.cview, 0, (words + 1) * sizeof(uint2)));
+        CK(dalloc(&s.word_epoch, words));
+        CK(cudaMemset(s.word_epoch, 0, words * 4));
+        CK(cudaMemset(s.pstate, 0, sizeof(PartState)));  // the stamps start over
+        CK(cudaStreamSynchronize(cudaStreamLegacy));
+        ctx->scratch_gen++;
         ctx->alloc_words = words;
     }
     s.n_words = words;
@@ -120,6 +127,7 @@ int ensure_scratch(ltp_ctx *ctx, uint64_t n_ops) {
         CK(dalloc(&s.st_apply, tiles));
         CK(dalloc(&s.st_ins, tiles * LTP_MAX_TABLES));
         CK(dalloc(&s.ins_pre, tiles * LTP_MAX_TABLES));
+        ctx->scratch_gen++;
         s.cap_ops = cap;
         s.cap_tiles = tiles;
         s.cap_sort_tiles = stiles;
@@ -188,6 +196,12 @@ int ltp_init(const ltp_config *cfg, ltp_ctx **out) {
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->ctr, sizeof(Counters));
     if (e == cudaSuccess) e = cudaMemset(ctx->ctr, 0, sizeof(Counters));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->s.pctr, 2 * sizeof(PartCounters));
+    if (e == cudaSuccess) e = cudaMemset(ctx->s.pctr, 0, 2 * sizeof(PartCounters));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->s.fctr, sizeof(Counters));
+    if (e == cudaSuccess) e = cudaMemset(ctx->s.fctr, 0, sizeof(Counters));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->s.pstate, sizeof(PartState));
+    if (e == cudaSuccess) e = cudaMemset(ctx->s.pstate, 0, sizeof(PartState));
     if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->rows_now, LTP_MAX_TABLES * sizeof(u64));
     if (e == cudaSuccess) e = cudaMemset(ctx->rows_now, 0, LTP_MAX_TABLES * sizeof(u64));
     if (e != cudaSuccess) {
@@ -213,6 +227,9 @@ int ltp_shutdown(ltp_ctx *ctx) {
     free_scratch_ops(ctx->s);
     free_scratch_words(ctx->s);
     cudaFree(ctx->ctr);
+    cudaFree(ctx->s.pctr);
+    cudaFree(ctx->s.fctr);
+    cudaFree(ctx->s.pstate);
     cudaFree(ctx->rows_now);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->p_exec) cudaGraphExecDestroy(ctx->p_exec);
@@ -258,6 +275,7 @@ int ltp_table_create_cap(ltp_ctx *ctx, const ltp_schema *schema, uint64_t rows, 
     t.dev.n_cols = schema->n_cols;
     t.dev.cell_base = ctx->total_cells;
     t.dev.wide = schema->wide_cols;
+    t.dev.inv = t.n_cols > 1 ? ~0ull / t.n_cols + 1ull : 0ull;
     t.bytes = col_off(t.dev, schema->n_cols);  // offset one past the last column
     CK(cudaMalloc((void **)&t.dev.data, t.bytes));
     CK(cudaMemset(t.dev.data, 0, t.bytes));
@@ -506,8 +524,6 @@ BatchDev batch_dev(const ltp_batch *b) {
 
 // Stream-ordered launches of one batch (scratch already sized and clean).
 int execute_one(ltp_ctx *ctx, ltp_batch *b, cudaStream_t st, bool allow_stall) {
-    CK(cudaMemsetAsync(ctx->ctr, 0, sizeof(Counters), st));
-    if (b->n_txns) CK(cudaMemsetAsync(b->commit, 1, b->n_txns, st));
     Launch L;
     L.stream = st;
     L.num_sms = ctx->num_sms;
@@ -520,7 +536,21 @@ int execute_one(ltp_ctx *ctx, ltp_batch *b, cudaStream_t st, bool allow_stall) {
     L.ev = b->ev;
     L.progress = b->progress;
     L.progress_stage = b->progress_stage;
-    if (b->n_ops) CK(launch_execute(L, batch_dev(b), tables_dev(ctx), ctx->s, ctx->ctr));
+    const BatchDev bd = batch_dev(b);
+    const TablesDev T = tables_dev(ctx);
+    cudaError_t e = cudaSuccess;
+    if (launch_buckets(L, bd, T, ctx->s, b->snap, &e)) {
+        if (e != cudaSuccess) {
+            ctx->dirty = true;
+            return cuda_fail(ctx, e, "bucket kernels");
+        }
+        b->rule = ctx->rule;
+        b->executed = true;
+        return LTP_OK;
+    }
+    CK(cudaMemsetAsync(ctx->ctr, 0, sizeof(Counters), st));
+    if (b->n_txns) CK(cudaMemsetAsync(b->commit, 1, b->n_txns, st));
+    if (b->n_ops) CK(launch_execute(L, bd, T, ctx->s, ctx->ctr));
     CK(cudaMemcpyAsync(b->snap, ctx->ctr, sizeof(Counters), cudaMemcpyDeviceToDevice, st));
     b->rule = ctx->rule;
     b->executed = true;
@@ -599,6 +629,7 @@ int ltp_batches_execute(ltp_ctx *ctx, ltp_batch *const *batches, uint32_t n, int
         }
         key.push_back(ctx->tables.size());
         key.push_back(ctx->any_wide ? 1u : 0u);
+        key.push_back(ctx->scratch_gen);
         if (!ctx->graph_exec || key != ctx->graph_key) {
             if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
             ctx->graph_exec = nullptr;
@@ -629,7 +660,7 @@ int ltp_batches_execute(ltp_ctx *ctx, ltp_batch *const *batches, uint32_t n, int
     // persistent: one cooperative kernel over all batches.  The batch
     // descriptors stay on the device while the list is unchanged, and the
     // launch (counter reset + cooperative kernel) is a captured CUDA graph.
-    std::vector<uint64_t> key = {(uint64_t)ctx->rule, ctx->tables.size(), ctx->any_wide ? 1u : 0u};
+    std::vector<uint64_t> key = {(uint64_t)ctx->rule, ctx->tables.size(), ctx->any_wide ? 1u : 0u, ctx->scratch_gen};
     for (uint32_t i = 0; i < n; i++) {
         const ltp_batch *b = batches[i];
         key.insert(key.end(), {(uint64_t)(uintptr_t)b, b->n_ops, b->n_txns, b->ops_per_txn,
@@ -894,7 +925,7 @@ static int pipe_execute(ltp_ctx *ctx, PipeSlot &sl, cudaStream_t sx) {
                                        ((uint64_t)t.word_bits << 32) | t.flags, (uint64_t)b->key32,
                                        (uint64_t)ctx->rule,
                                        (uint64_t)(b->have_events && (ctx->flags & LTP_FLAG_STAGE_TIMING)),
-                                       ctx->tables.size(), ctx->any_wide ? 1u : 0u};
+                                       ctx->tables.size(), ctx->any_wide ? 1u : 0u, ctx->scratch_gen};
     if (sl.gexec && key == sl.gkey) {
         CK(cudaGraphLaunch(sl.gexec, sx));
         sl.b->rule = ctx->rule;

@@ -39,6 +39,7 @@ struct ltp_ctx {
     bool any_wide = false;  // some table has an int64 column
     Scratch s;
     uint64_t alloc_words = 0;  // bitmap words currently allocated
+    uint64_t scratch_gen = 0;  // counts scratch allocations: captured launches hold scratch pointers
     Counters *ctr = nullptr;
     u64 *rows_now = nullptr;  // [LTP_MAX_TABLES] device row counts
     std::string last_error;

@@ -32,6 +32,7 @@ struct TableDev {
     u64 wide;       // bit c: column c holds int64
     u32 n_cols;
     u32 pad;
+    u64 inv;        // ceil(2^64 / n_cols) (n_cols > 1): divides a 32-bit cell number by n_cols
 };
 
 __host__ __device__ __forceinline__ u64 col_off(const TableDev &t, u32 c) {
@@ -104,6 +105,27 @@ struct __align__(16) WordState {
     u32 pad;     // keeps a word to one 16-byte access (the dense ids live in Scratch::cview)
 };
 
+// Device state of the bucket path (ltp_buckets.cu) that outlives a batch.
+// Its counters are double-buffered: a batch uses PartCounters [par], which is
+// zero, and its first kernel clears the other one for the next batch.  The
+// values a batch starts from (stamp1, par1) are written by its last kernel
+// that reads stamp2, par2, and the other way round, so no kernel writes what
+// its other blocks read.
+struct PartState {
+    u32 stamp1, par1;
+    u32 stamp2, par2;  // stamp: batches executed, marks the conflict words a batch touched
+    u32 skew;          // the batch at hand has an overlong bucket: left to the conflict-word path
+    u32 full;          // the batch at hand found no room for its inserts
+    u32 bar[2];        // grid barrier of the fallback launch
+};
+constexpr u32 kMaxBuckets = 1536;  // four waves and more of two blocks per SM
+struct PartCounters {
+    Counters c;              // err, bad_op and the insert counts
+    u32 writes;              // some op writes an existing cell
+    u32 hot;                 // some bucket has long runs ...
+    u32 total[kMaxBuckets];  // ... this many records of them per bucket
+};
+
 // Scratch owned by the context, sized by the cell space and the batch capacity.
 struct Scratch {
     WordState *words; // [n_words]
@@ -118,6 +140,13 @@ struct Scratch {
     u64 *st_apply;  // [tiles] segmented-apply look-back status
     u32 *st_ins;    // [tiles * LTP_MAX_TABLES] insert-slot look-back status
     u32 *ins_pre;   // [tiles * LTP_MAX_TABLES] per insert tile and table: insert ops (mark), then their exclusive prefix
+    // bucket path (null: not available): its counters [2], its state, clean
+    // counters for the fallback, and per conflict word the stamp of the last
+    // batch that touched it
+    PartCounters *pctr;
+    Counters *fctr;
+    PartState *pstate;
+    u32 *word_epoch;
     u64 n_words;
     u64 cap_ops;
     u64 cap_tiles;  // tiles of the smallest look-back tile size at cap_ops
@@ -161,6 +190,17 @@ struct Launch {
 // Kernel launch wrappers (ltp_kernels.cu).  Each returns the CUDA status of
 // its launches.
 cudaError_t launch_execute(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr);
+// The bucket path (ltp_buckets.cu): launches the whole batch, counters and
+// snapshot included, and returns true, or returns false for a batch it does
+// not take.
+bool launch_buckets(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *snap,
+                    cudaError_t *status);
+// Pieces of the conflict-word path that the bucket path uses: the insert
+// kernel, and the persistent kernel on one batch, run only when
+// s.pstate->skew is set.
+cudaError_t launch_insert(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
+                          int prefixed, const PartState *ps);
+cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *snap);
 // Is (threads per block, ops per thread, conflict-word bits) a built tiling?
 bool tiling_supported(int block, int ipt, int word_bits);
 cudaError_t launch_reset_scratch(cudaStream_t st, const Scratch &s);
