@@ -36,7 +36,8 @@ struct TableDev {
 };
 
 __host__ __device__ __forceinline__ u64 col_off(const TableDev &t, u32 c) {
-    const u64 below = c ? (t.wide & ((1ull << c) - 1ull)) : 0ull;
+    // (c = 64, one past the last of 64 columns: every wide column; a shift by 64 is undefined)
+    const u64 below = c >= 64 ? t.wide : t.wide & ((1ull << c) - 1ull);
 #ifdef __CUDA_ARCH__
     const u32 nw = __popcll(below);
 #else
