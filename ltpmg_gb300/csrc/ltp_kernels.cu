@@ -1197,8 +1197,7 @@ constexpr u32 kInsSmemDesc = kInsSmem + kInsPairs * 8 + (kInsPairs + 1) * 4 + kI
 static_assert(kInsSmem % 8 == 0, "the descriptors' addresses start 8-byte aligned");
 
 template <int BLK, bool DESC>
-__device__ __forceinline__ void phase_insert(const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
-                                             bool prefixed) {
+__device__ __forceinline__ void phase_insert(const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr) {
     constexpr u32 IIPT = kInsTile / BLK;
     if (block_err(ctr)) return;
     u32 any = 0;
@@ -1240,7 +1239,7 @@ __device__ __forceinline__ void phase_insert(const BatchDev &b, const TablesDev 
                 const u32 w = b.opw[i];
                 if (opw_kind(w) == LTP_OP_INSERT) {
                     t = opw_table(w);
-                    ins = prefixed || b.commit[op_tid(b, i)] != 0;  // prefixed: every transaction commits
+                    ins = b.commit[op_tid(b, i)] != 0;
                     if (!ins) store_out(b, i, 0);
                 }
             }
@@ -1264,11 +1263,7 @@ __device__ __forceinline__ void phase_insert(const BatchDev &b, const TablesDev 
             u32 *st = s.st_ins;
             u32 excl = 0;
             u32 *slot = &st[(u64)tile * LTP_MAX_TABLES + t];
-            if (prefixed) {
-                // every transaction commits (ordered rule): the tile's offset
-                // is the prefix of the insert counts mark took, no look-back
-                excl = s.ins_pre[(u64)tile * LTP_MAX_TABLES + t];
-            } else if (tile == 0) {
+            if (tile == 0) {
                 st_status32(slot, (2u << 30) | run);
             } else {
                 st_status32(slot, (1u << 30) | run);
@@ -1393,14 +1388,9 @@ __device__ __forceinline__ void phase_insert(const BatchDev &b, const TablesDev 
     }
 }
 
-__global__ void __launch_bounds__(kInsBlock) k_insert(BatchDev b, TablesDev T, Scratch s, Counters *ctr, int prefixed,
-                                                      const PartState *ps) {
+__global__ void __launch_bounds__(kInsBlock) k_insert(BatchDev b, TablesDev T, Scratch s, Counters *ctr) {
     pdl_begin();
-    if (ps) {  // bucket path: its current counters; nothing to do for a batch it left or refused
-        if (ps->skew || ps->full) return;
-        ctr = &s.pctr[ps->par2].c;
-    }
-    phase_insert<kInsBlock, true>(b, T, s, ctr, prefixed != 0);
+    phase_insert<kInsBlock, true>(b, T, s, ctr);
 }
 
 // Ordered rule: every insert commits, so the rank of an insert among its
@@ -1437,6 +1427,235 @@ __global__ void __launch_bounds__(kInsPrefixBlock) k_ins_prefix(BatchDev b, Tabl
             pre += c;
         }
         __syncthreads();  // s_wsum is reused by the next table
+    }
+}
+
+// Committed inserts under the ordered rule, where every transaction commits
+// and the offsets of the 4096-op insert tiles are known: half a tile per
+// block.  New rows go from the payload's rows to the tables' columns through
+// shared memory: requested as they lie in the payload (consecutive lanes,
+// consecutive slots; cp.async, so that all of a block's rows are under way
+// at once) and written column by column (consecutive lanes, consecutive
+// rows).  Bound by the latency of its chain (opwords, keys, rows, links) and
+// by the row reads.  Reading every cell straight from its row, a sector per 4
+// bytes, the insert kernel took 76 us for 1.38 M order-entry ops, 26 us for
+// 1.8 M YCSB-E ops and 39 us for the 31,500 ops of a small order-entry call;
+// this one 47, 22 and 17 us (512 threads x 4 ops, two blocks per SM; 256 x 8
+// with three: 3% slower on order entry, 3% faster on YCSB-E).
+constexpr u32 kRowsBlock = 512, kRowsIpt = 4, kRowsTile = kRowsBlock * kRowsIpt;
+constexpr u32 kRowsStage = 11264;  // 4-byte slots staged at a time
+constexpr u32 kRowsSmem = kRowsStage * 4 + kRowsTile * 4;
+static_assert(kInsTile == 2 * kRowsTile, "an insert tile is two of these");
+static_assert(kRowsStage >= 2 * LTP_MAX_COLS * 3, "a row and its padding fit");
+
+__device__ __forceinline__ void copy_async4(u32 *dst, const int32_t *src) {
+    const u32 d = (u32)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__global__ void __launch_bounds__(kRowsBlock, 2) k_rows(BatchDev b, TablesDev T, Scratch s, Counters *ctr,
+                                                        const PartState *ps) {
+    pdl_begin();
+    if (ps) {  // bucket path: its current counters; nothing to do for a batch it left or refused
+        if (ps->skew || ps->full) return;
+        ctr = &s.pctr[ps->par2].c;
+    }
+    if (block_err(ctr)) return;
+    constexpr int NW = kRowsBlock / 32;
+    constexpr u32 G = kRowsIpt * NW;  // groups of 32 consecutive ops
+    const u32 tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    u32 *s_stage = ltp_dyn_smem;          // [kRowsStage]
+    u32 *s_off = s_stage + kRowsStage;    // [kRowsTile] payload offset of every new row, by table and rank
+    __shared__ u32 s_cnt[LTP_MAX_TABLES][G];  // inserts per table and group, then their exclusive sums
+    __shared__ u32 s_half[LTP_MAX_TABLES], s_tot[LTP_MAX_TABLES], s_toff[LTP_MAX_TABLES], s_slots[LTP_MAX_TABLES];
+    __shared__ u32 s_at[LTP_MAX_TABLES], s_r0[LTP_MAX_TABLES], s_take[LTP_MAX_TABLES];  // the staged rows of each table
+    __shared__ u32 s_mask;
+    __shared__ u64 s_base[LTP_MAX_TABLES], s_wide[LTP_MAX_TABLES];
+    if (tid < LTP_MAX_TABLES) {
+        s_wide[tid] = tid < T.n ? T.t[tid].wide : 0ull;
+        s_slots[tid] = tid < T.n ? (u32)insert_slots(T.t[tid]) : 1u;
+    }
+    if (tid < 32) {
+        const u32 m = __ballot_sync(FULL_MASK, tid < T.n && ctr->ins_total[tid < T.n ? tid : 0] != 0u);
+        if (tid == 0) s_mask = m;
+    }
+    __syncthreads();
+    const u32 mask = s_mask;  // tables that gain rows
+    if (!mask) return;
+    const u64 n = b.n_ops;
+    const u64 slices = (n + kRowsTile - 1) / kRowsTile;
+    for (u64 slice = blockIdx.x; slice < slices; slice += gridDim.x) {
+        const u64 base = slice * kRowsTile;
+        u32 w[kRowsIpt];
+#pragma unroll
+        for (int k = 0; k < (int)kRowsIpt; k++) {
+            const u64 i = base + (u32)k * kRowsBlock + tid;
+            w[k] = i < n ? b.opw[i] : 0u;
+        }
+        if (tid < LTP_MAX_TABLES) s_half[tid] = s_tot[tid] = 0u;
+        __syncthreads();
+        if (slice & 1u) {  // the inserts of the tile's first half
+            u32 h[kRowsIpt];
+#pragma unroll
+            for (int k = 0; k < (int)kRowsIpt; k++) h[k] = b.opw[base - kRowsTile + (u32)k * kRowsBlock + tid];
+            for (u32 m = mask; m; m &= m - 1) {
+                const u32 t = (u32)__ffs(m) - 1u;
+                u32 c = 0;
+#pragma unroll
+                for (int k = 0; k < (int)kRowsIpt; k++)
+                    c += (u32)__popc(__ballot_sync(FULL_MASK, opw_kind(h[k]) == LTP_OP_INSERT && opw_table(h[k]) == t));
+                if (lane == 0 && c) atomicAdd(&s_half[t], c);
+            }
+        }
+        // each insert's rank among its table's, in op order
+        u32 rank[kRowsIpt];
+        for (u32 m = mask; m; m &= m - 1) {
+            const u32 t = (u32)__ffs(m) - 1u;
+#pragma unroll
+            for (int k = 0; k < (int)kRowsIpt; k++) {
+                const bool mine = opw_kind(w[k]) == LTP_OP_INSERT && opw_table(w[k]) == t;
+                const u32 bal = __ballot_sync(FULL_MASK, mine);
+                if (mine) rank[k] = (u32)__popc(bal & lanemask_lt());
+                if (lane == 0) s_cnt[t][k * NW + warp] = (u32)__popc(bal);
+            }
+        }
+        __syncthreads();
+        for (u32 t = warp; t < LTP_MAX_TABLES; t += NW) {  // a warp per table
+            if (!(mask >> t & 1u)) continue;
+            u32 x[G / 32], sum = 0;
+#pragma unroll
+            for (int j = 0; j < (int)(G / 32); j++) {
+                x[j] = s_cnt[t][lane * (G / 32) + j];
+                sum += x[j];
+            }
+            u32 incl = sum;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const u32 y = __shfl_up_sync(FULL_MASK, incl, d);
+                if (lane >= d) incl += y;
+            }
+            u32 run = incl - sum;
+#pragma unroll
+            for (int j = 0; j < (int)(G / 32); j++) {
+                s_cnt[t][lane * (G / 32) + j] = run;
+                run += x[j];
+            }
+            if (lane == 31) {
+                s_tot[t] = incl;
+                if (incl) {
+                    s_base[t] = T.rows_now[t] + s.ins_pre[(base / kInsTile) * LTP_MAX_TABLES + t] + s_half[t];
+                    atomicAdd(&ctr->ins_committed[t], incl);
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < LTP_MAX_TABLES) {
+            u32 off = 0;
+            for (u32 t = 0; t < tid; t++) off += s_tot[t];
+            s_toff[tid] = off;
+        }
+        u32 off[kRowsIpt];
+#pragma unroll
+        for (int k = 0; k < (int)kRowsIpt; k++)
+            off[k] = opw_kind(w[k]) == LTP_OP_INSERT ? (u32)op_key(b, base + (u32)k * kRowsBlock + tid) : 0u;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < (int)kRowsIpt; k++)
+            if (opw_kind(w[k]) == LTP_OP_INSERT) {
+                const u64 i = base + (u32)k * kRowsBlock + tid;
+                const u32 t = opw_table(w[k]);
+                rank[k] += s_cnt[t][k * NW + warp];
+                s_off[s_toff[t] + rank[k]] = off[k];
+                store_out(b, i, (long long)(s_base[t] + rank[k]));
+            }
+        // the rows, as many at a time as the stage holds (usually all)
+        u32 ct = 0, cr = 0;  // the next row
+        while (ct < LTP_MAX_TABLES) {
+            if (tid < LTP_MAX_TABLES) s_take[tid] = 0u;
+            __syncthreads();
+            u32 used = 0;
+            while (ct < LTP_MAX_TABLES) {
+                if (cr == s_tot[ct]) {
+                    ct++;
+                    cr = 0;
+                    continue;
+                }
+                const u32 slots = s_slots[ct], left = s_tot[ct] - cr, fit = (kRowsStage - used) / slots;
+                u32 take = min(left, fit);
+                if (take && ((take | 1u) > fit)) take--;  // an odd pitch keeps a row's slots in different banks
+                if (take == 0) break;
+                const u32 pitch = take | 1u;
+                if (tid == 0) {
+                    s_at[ct] = used;
+                    s_r0[ct] = cr;
+                    s_take[ct] = take;
+                }
+                // lanes of a row: the power of two that covers its slots
+                const u32 lg = slots > 16 ? 5u : slots > 8 ? 4u : slots > 4 ? 3u : 2u;
+                const u32 sub = lane & ((1u << lg) - 1u), per = 32u >> lg;
+                const u32 *row_off = s_off + s_toff[ct] + cr;
+                for (u32 r = warp * per + ((u32)lane >> lg); r < take; r += NW * per) {
+                    const int32_t *src = b.payload + row_off[r];
+                    u32 *dst = s_stage + used + r;
+                    for (u32 c = sub; c < slots; c += 1u << lg) copy_async4(dst + c * pitch, src + c);
+                }
+                used += slots * pitch;
+                cr += take;
+                if (cr < s_tot[ct]) break;  // full (a table has one run of rows in the stage)
+            }
+            // linked columns take their op's output, read while the rows come
+            // in: each step's loads are requested for all the thread's ops
+            long long lv[kRowsIpt];
+            u32 lw[kRowsIpt];
+#pragma unroll
+            for (int k = 0; k < (int)kRowsIpt; k++) {
+                const u32 d = opw_kind(w[k]) == LTP_OP_INSERT ? insert_link(w[k]) : 0u;
+                lw[k] = d ? b.opw[base + (u32)k * kRowsBlock + tid - d] : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < (int)kRowsIpt; k++) {
+                const u64 i = base + (u32)k * kRowsBlock + tid;
+                const u32 d = opw_kind(w[k]) == LTP_OP_INSERT ? insert_link(w[k]) : 0u;
+                const bool wide = b.out64 && (s_wide[opw_table(lw[k])] >> opw_col(lw[k]) & 1ull);
+                lv[k] = !d ? 0ll : wide ? b.out64[i - d] : (long long)b.out[i - d];
+            }
+            copy_async_wait();
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < (int)kRowsIpt; k++)
+                if (opw_kind(w[k]) == LTP_OP_INSERT && insert_link(w[k])) {
+                    const u32 t = opw_table(w[k]), r = rank[k] - s_r0[t];
+                    if (s_take[t] && rank[k] >= s_r0[t] && r < s_take[t]) {
+                        const u32 col = opw_col(w[k]), pitch = s_take[t] | 1u;
+                        const u64 wd = s_wide[t];
+                        u32 *dst = s_stage + s_at[t] + r + (col + (u32)__popcll(wd & ((1ull << col) - 1ull))) * pitch;
+                        dst[0] = (u32)(u64)lv[k];
+                        if (wd >> col & 1ull) dst[pitch] = (u32)((u64)lv[k] >> 32);
+                    }
+                }
+            __syncthreads();
+            for (u32 m = mask; m; m &= m - 1) {
+                const u32 t = (u32)__ffs(m) - 1u, take = s_take[t], pitch = take | 1u;
+                if (!take) continue;
+                const TableDev &tab = T.t[t];
+                const u64 wd = s_wide[t], row0 = s_base[t] + s_r0[t];
+                for (u32 c = warp; c < tab.n_cols; c += NW) {  // a warp per column
+                    const u32 *src = s_stage + s_at[t] + (c + (u32)__popcll(wd & ((1ull << c) - 1ull))) * pitch;
+                    char *dst = tab.data + col_off(tab, c);
+                    if (wd >> c & 1ull) {
+                        for (u32 j = lane; j < take; j += 32)
+                            if (LTP_IN_BOUNDS(ctr, row0 + j, tab.rows_cap))
+                                reinterpret_cast<u64 *>(dst)[row0 + j] = (u64)src[pitch + j] << 32 | src[j];
+                    } else {
+                        for (u32 j = lane; j < take; j += 32)
+                            if (LTP_IN_BOUNDS(ctr, row0 + j, tab.rows_cap)) reinterpret_cast<u32 *>(dst)[row0 + j] = src[j];
+                    }
+                }
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -1636,6 +1855,17 @@ static int capped(int grid, u64 upper) { return (int)((u64)grid < upper ? (u64)g
 
 cudaError_t launch_insert(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
                           int prefixed, const PartState *ps) {
+    if (prefixed) {
+        static int grows = 0, rsms = 0;
+        if (rsms != L.num_sms) {
+            const cudaError_t e = cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
+            if (e != cudaSuccess) return e;
+            grows = occ_grid(k_rows, (int)kRowsBlock, L.num_sms, kRowsSmem);
+            rsms = L.num_sms;
+        }
+        return launch_k(L.pdl, k_rows, capped(grows, (b.n_ops + kRowsTile - 1) / kRowsTile), kRowsBlock, kRowsSmem, L.stream, b,
+                        T, s, ctr, ps);
+    }
     static int gins = 0, sms = 0;
     if (sms != L.num_sms) {
         const cudaError_t e = cudaFuncSetAttribute(k_insert, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInsSmemDesc);
@@ -1644,7 +1874,7 @@ cudaError_t launch_insert(const Launch &L, const BatchDev &b, const TablesDev &T
         sms = L.num_sms;
     }
     return launch_k(L.pdl, k_insert, capped(gins, (b.n_ops + kInsTile - 1) / kInsTile), kInsBlock, kInsSmemDesc, L.stream,
-                    b, T, s, ctr, prefixed, ps);
+                    b, T, s, ctr);
 }
 
 cudaError_t launch_execute(const Launch &L_in, const BatchDev &b_in, const TablesDev &T, const Scratch &s,
@@ -1839,7 +2069,7 @@ __global__ void __launch_bounds__(kPBlock, 2) k_persist(PersistArgs a) {
         }
         grid_sync(a.bar, nb, a.ctr);
         if (b.payload_len) {  // a batch without payload has no valid insert
-            phase_insert<kPBlock, false>(b, a.T, a.s, a.ctr, false);
+            phase_insert<kPBlock, false>(b, a.T, a.s, a.ctr);
             grid_sync(a.bar, nb, a.ctr);
         }
         phase_finish<32>(b, a.T, a.s, a.ctr, a.rule);

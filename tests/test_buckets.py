@@ -132,3 +132,41 @@ def test_refused_batches_change_nothing(lib_loaded, n_ops):
         _, vals, _ = b.results()
         ref, _, ro = O.replay(0, ref, np.arange(n_ops + 1, dtype=np.uint32), keys, opw)
         assert np.array_equal(vals, ro) and np.array_equal(ctx.download(t), ref)
+
+
+@pytest.mark.parametrize("n_txns", [1, 700, 1024, 5000])
+def test_rows_of_every_width(lib_loaded, n_txns):
+    """Inserts into tables of 1 to 64 columns, int32 and int64, linked and
+    not, in batches whose new rows need one staging or several."""
+    rng = np.random.default_rng(n_txns)
+    shapes = [(64, 0), (3, 0b010), (64, (1 << 64) - 1), (1, 0), (17, 1 << 16)]  # columns, int64 ones
+    slots = [c + bin(m).count("1") for c, m in shapes]
+    t = rng.integers(0, len(shapes), n_txns)
+    t[: n_txns // 2] = 2  # the widest rows, together
+    col = np.array([rng.integers(0, shapes[x][0]) for x in t])
+    link = rng.random(n_txns) < 0.5
+    first = np.concatenate([[0], np.cumsum(np.array(slots)[t])])
+    # a transaction: one read-modify-write of table 0, one insert that may take its output
+    keys = np.stack([rng.integers(0, 50, n_txns), first[:-1]], axis=1).reshape(-1).astype(np.uint64)
+    add = [G.opword(G.OP_ADD, int(c), 0, int(v)) for c, v in zip(rng.integers(0, 64, n_txns), rng.integers(-99, 99, n_txns))]
+    ins = [G.opword(G.OP_INSERT, int(c), int(x), int(li)) for c, x, li in zip(col, t, link)]
+    opw = np.stack([add, ins], axis=1).reshape(-1).astype(np.uint32)
+    pay = rng.integers(-(1 << 31), 1 << 31, int(first[-1])).astype(np.int32)
+    tf = np.arange(0, 2 * n_txns + 1, 2, dtype=np.uint32)
+    rows = [50 + int((t == k).sum()) for k in range(len(shapes))]
+    with G.Context(device=0) as ctx:
+        for k, (c, m) in enumerate(shapes):
+            ctx.create_table(50, c, rows_cap=rows[k], wide=[j for j in range(c) if m >> j & 1])
+            ctx.fill_seeded(k, 11)
+        tabs = [(np.concatenate([ctx.download(k), np.zeros((c, rows[k] - 50), np.int64 if m else np.int32)], axis=1), 50, m)
+                for k, (c, m) in enumerate(shapes)]
+        b = ctx.batch(n_txns, len(keys))
+        b.load(tf, keys, opw)
+        b.load_payload(pay)
+        b.execute()
+        _, vals, _ = b.results64()
+        finals = [ctx.download(k) for k in range(len(shapes))]
+    after, _, ro = O.replay_tables(0, tabs, tf, keys, opw, pay)
+    assert np.array_equal(vals, ro)
+    for k in range(len(shapes)):
+        assert np.array_equal(finals[k], after[k][0][:, :after[k][1]]), k
