@@ -1079,12 +1079,13 @@ __global__ void __launch_bounds__(kApplyBlock, 4) k_apply_auto(BatchDev b, Table
 // The first kernel notes every op's contended id (or none), so that the other
 // two read a word in op order where they would look the cell's view up again;
 // it and the second take four ops of a thread at a time, their loads
-// requested together.  2.1 M ops, Zipf 0.7: 57 -> 21, 19 -> 8 and 32 -> 30 us.
-constexpr int kR1Ipt = 4;
+// requested together (one at a time in batches that would leave threads
+// without an op: 48,000 ops 38 and 40 us a batch).  2.1 M ops, Zipf 0.7:
+// 57 -> 21, 19 -> 8 and 32 -> 30 us.
 constexpr u32 kNoId = 0xFFFFFFFFu;
 __device__ __forceinline__ u32 *r1_ids(const Scratch &s) { return reinterpret_cast<u32 *>(s.list[0]); }
 
-template <int WB>
+template <int WB, int kR1Ipt>
 __device__ __forceinline__ void phase_r1_minw(const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr) {
     if (block_err(ctr)) return;
     const u64 n = b.n_ops, span = (u64)blockDim.x * kR1Ipt;
@@ -1132,12 +1133,13 @@ __device__ __forceinline__ void phase_r1_minw(const BatchDev &b, const TablesDev
     if (threadIdx.x == 0 && s_count) atomicAdd(&ctr->n_c, (u64)s_count);
 }
 
-template <int WB>
+template <int WB, int IPT>
 __global__ void __launch_bounds__(256) k_r1_minw(BatchDev b, TablesDev T, Scratch s, Counters *ctr) {
     pdl_begin();
-    phase_r1_minw<WB>(b, T, s, ctr);
+    phase_r1_minw<WB, IPT>(b, T, s, ctr);
 }
 
+template <int kR1Ipt>
 __device__ __forceinline__ void phase_r1_abort(const BatchDev &b, const Scratch &s, Counters *ctr) {
     if (block_err(ctr)) return;
     const u64 n = b.n_ops, span = (u64)blockDim.x * kR1Ipt;
@@ -1160,9 +1162,10 @@ __device__ __forceinline__ void phase_r1_abort(const BatchDev &b, const Scratch 
     }
 }
 
+template <int IPT>
 __global__ void __launch_bounds__(256) k_r1_abort(BatchDev b, TablesDev T, Scratch s, Counters *ctr) {
     pdl_begin();
-    phase_r1_abort(b, s, ctr);
+    phase_r1_abort<IPT>(b, s, ctr);
 }
 
 // (one op per thread at a time, eight blocks per SM: with two ops, and with
@@ -1985,9 +1988,10 @@ cudaError_t launch_execute(const Launch &L_in, const BatchDev &b_in, const Table
         chk(launch_k(L.pdl, T.any_wide ? k_apply_auto : k_apply<u32>, gapp, kApplyBlock, 0, L.stream, b, T, s, ctr));
         mark_ev(8);
     } else {
-        chk(launch_k(L.pdl, wide_words ? k_r1_minw<64> : k_r1_minw<32>, gstream, 256, 0, L.stream, b, T, s, ctr));
+        const bool many = b.n_ops >= 4ull * gstream * 256;
+        chk(launch_k(L.pdl, wide_words ? (many ? k_r1_minw<64, 4> : k_r1_minw<64, 1>) : (many ? k_r1_minw<32, 4> : k_r1_minw<32, 1>), gstream, 256, 0, L.stream, b, T, s, ctr));
         mark_ev(3);
-        chk(launch_k(L.pdl, k_r1_abort, gstream, 256, 0, L.stream, b, T, s, ctr));
+        chk(launch_k(L.pdl, many ? k_r1_abort<4> : k_r1_abort<1>, gstream, 256, 0, L.stream, b, T, s, ctr));
         mark_ev(4);
         chk(launch_k(L.pdl, k_r1_exec, gstream, 256, 0, L.stream, b, T, s, ctr));
         for (int i = 5; i <= 8; i++) mark_ev(i);
@@ -2098,9 +2102,9 @@ __global__ void __launch_bounds__(kPBlock, 2) k_persist(PersistArgs a) {
             if (a.T.any_wide && *(volatile u32 *)&a.ctr->wide_ops) phase_apply<kPBlock, u64>(b, a.T, a.s, a.ctr);
             else phase_apply<kPBlock, u32>(b, a.T, a.s, a.ctr);
         } else {
-            phase_r1_minw<32>(b, a.T, a.s, a.ctr);
+            phase_r1_minw<32, 1>(b, a.T, a.s, a.ctr);
             grid_sync(a.bar, nb, a.ctr);
-            phase_r1_abort(b, a.s, a.ctr);
+            phase_r1_abort<1>(b, a.s, a.ctr);
             grid_sync(a.bar, nb, a.ctr);
             phase_r1_exec(b, a.T, a.s, a.ctr);
         }
