@@ -230,14 +230,14 @@ __global__ void __launch_bounds__(kPartBlock, 3) k_part(BatchDev b, TablesDev T,
     u64 rec[IPT];
     u32 bk[IPT];  // bucket, then bucket | rank << 16; ~0: no record
     bool any = false;
+    u32 ins = 0;
 #pragma unroll
     for (int k = 0; k < IPT; k++) {
         const u64 i = wbase + (u64)k * 32 + lane;
         bk[k] = 0xFFFFFFFFu;
         if (i >= n) continue;
         if (opw_kind(w[k]) == LTP_OP_INSERT) {
-            if (insert_valid(b, T, key[k], i, w[k])) atomicAdd(&s_ins[opw_table(w[k])], 1u);
-            else set_bad(&pc->c, i);
+            ins |= 1u << k;
             continue;
         }
         u32 cell;
@@ -250,6 +250,35 @@ __global__ void __launch_bounds__(kPartBlock, 3) k_part(BatchDev b, TablesDev T,
         any |= add != 0u;
         bk[k] = (u32)__umul64hi((u64)h, p.width_inv);
         rec[k] = ((u64)h << 32) | (u64)(add << 31 | (add ? (w[k] >> 12) << kOpBits : 0u) | (u32)(i - base));
+    }
+    if (__any_sync(FULL_MASK, ins != 0u)) {
+        // inserts: a link must name a read or read-modify-write before it in
+        // its transaction.  Each of the three loads that takes is requested
+        // for all rows at once (one row after another, they took a third of
+        // the kernel on order entry).
+        u32 tid_[IPT], linked[IPT], first[IPT];
+#pragma unroll
+        for (int k = 0; k < IPT; k++) {
+            const u64 i = wbase + (u64)k * 32 + lane;
+            const u32 d = ins >> k & 1u ? insert_link(w[k]) : 0u;
+            tid_[k] = d ? op_tid(b, i) : 0u;
+            linked[k] = d && d <= i ? b.opw[i - d] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < IPT; k++) {
+            const bool on = (ins >> k & 1u) && insert_link(w[k]);
+            first[k] = !on ? 0u : b.ops_per_txn ? tid_[k] * b.ops_per_txn : b.txn_first[tid_[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < IPT; k++)
+            if (ins >> k & 1u) {
+                const u64 i = wbase + (u64)k * 32 + lane;
+                const u32 tb = opw_table(w[k]), d = insert_link(w[k]);
+                bool ok = tb < T.n && key[k] + insert_slots(T.t[tb]) <= b.payload_len;
+                if (ok && d) ok = opw_col(w[k]) < T.t[tb].n_cols && d <= i && i - d >= first[k] && opw_kind(linked[k]) <= LTP_OP_ADD;
+                if (ok) atomicAdd(&s_ins[tb], 1u);
+                else set_bad(&pc->c, i);
+            }
     }
     if (__any_sync(FULL_MASK, any) && lane == 0) s_any = 1u;
     // rank inside (warp, bucket), in op order: rows of 32 ops one after
@@ -366,7 +395,7 @@ struct Cfg {
     static constexpr u32 VB = WIDE ? 8 : 4;
     static constexpr u32 O_VAL = 0, O_CL = O_VAL + HS * VB, O_TAB = O_CL + 2 * CHUNK * 8, O_CNT = O_TAB + HS * 4,
                          O_OP = O_CNT + NW * ND * 4, BYTES_SOLO = O_OP, O_PRE = O_OP + CHUNK * 4,
-                         BYTES = O_PRE + (kMaxTiles + 1) * 4;
+                         BYTES = O_PRE + 2 * kMaxTiles * 4;
 };
 template <bool W>
 struct ValT {
@@ -381,8 +410,7 @@ struct ValT<true> {
 
 constexpr u32 kEmpty = 0xFFFFFFFFu;
 constexpr u32 kFew = 256;  // contended ops of a chunk that are resolved all against all
-constexpr u32 kHot = 192;  // ops on one cell that a long bucket scans for themselves ...
-constexpr u32 kHotCells = 8;  // ... for at most this many cells
+constexpr int kHotTries = 4;  // cells of a chunk with more that are scanned for themselves
 // slot word: cell number << 3 | these
 constexpr u32 kWritten = 1u, kMulti = 2u, kWideCell = 4u;
 
@@ -432,7 +460,8 @@ struct Smem {
     __device__ __forceinline__ u32 *tab() const { return reinterpret_cast<u32 *>(sm + C::O_TAB); }
     __device__ __forceinline__ u32 *cnt() const { return reinterpret_cast<u32 *>(sm + C::O_CNT); }
     __device__ __forceinline__ u32 *op() const { return reinterpret_cast<u32 *>(sm + C::O_OP); }    // ops of the staged records
-    __device__ __forceinline__ u32 *pre() const { return reinterpret_cast<u32 *>(sm + C::O_PRE); }  // [tiles + 1], long buckets
+    __device__ __forceinline__ u32 *pre() const { return reinterpret_cast<u32 *>(sm + C::O_PRE); }  // long buckets: [tiles],
+    __device__ __forceinline__ u32 *adj() const { return pre() + kMaxTiles; }                       // [tiles], see TileSrc
 };
 
 // Exclusive sums of a per-row, per-warp value (row-major: the order of the
@@ -597,6 +626,34 @@ __device__ __forceinline__ void run_sorted(const Smem<C> &m, const u32 rc, const
     }
 }
 
+// Executes rc <= kFew contended ops that cl holds in any order: each looks
+// at all of them, its cell's value is the sum over the ops on it up to its
+// own.  Returns the slot, and in *x the last value, of a cell whose last op is
+// this thread's, else kEmpty.
+template <class C>
+__device__ __forceinline__ u32 compare_all(const Smem<C> &m, const u32 rc, const BatchDev &b, Counters *ctr,
+                                           typename ValT<C::WIDE>::V *x) {
+    typedef typename ValT<C::WIDE>::V V;
+    typedef typename ValT<C::WIDE>::S S;
+    if (threadIdx.x >= rc) return kEmpty;
+    const u64 *cl = m.cl();
+    const u64 me = cl[threadIdx.x];
+    const u32 sl = (u32)(me >> 52), op = (u32)me;
+    u32 later = 0;
+    S sum = 0;
+#pragma unroll 8
+    for (u32 j = 0; j < rc; j++) {
+        const u64 o = cl[j];
+        const bool same = (u32)(o >> 52) == sl, upto = (u32)o <= op;
+        sum += same && upto ? (S)(V)imm20((u32)(o >> 32)) : (S)0;
+        later |= same && !upto;
+    }
+    const bool wd = C::WIDE && (m.tab()[sl] & kWideCell);
+    *x = narrow<C>((V)((S)m.val()[sl] + sum), wd);
+    put_out<C>(b, ctr, op, *x, wd);
+    return later ? kEmpty : sl;
+}
+
 // Executes the R <= CHUNK records that are staged (op order; kNoRec: none).
 // Adds this thread's share of the statistics.
 template <class C, class Src>
@@ -687,25 +744,9 @@ __device__ __forceinline__ void exec_chunk(const Src &src, const u32 R, const Ba
     };
     if (rc == 0) {
     } else if (rc <= kFew) {
-        // each looks at all of them: its cell's value is the sum over the
-        // ops on it up to its own
-        if (tid < rc) {
-            const u64 me = cl[tid];
-            const u32 sl = (u32)(me >> 52), op = (u32)me;
-            u32 later = 0;
-            S sum = 0;
-#pragma unroll 8
-            for (u32 j = 0; j < rc; j++) {
-                const u64 o = cl[j];
-                const bool same = (u32)(o >> 52) == sl, upto = (u32)o <= op;
-                sum += same && upto ? (S)(V)imm20((u32)(o >> 32)) : (S)0;
-                later |= same && !upto;
-            }
-            const bool wd = C::WIDE && (tab[sl] & kWideCell);
-            const V x = narrow<C>((V)((S)val[sl] + sum), wd);
-            put_out<C>(b, ctr, op, x, wd);
-            if (!later) store(sl, x);
-        }
+        V x = 0;
+        const u32 sl = compare_all<C>(m, rc, b, ctr, &x);
+        if (sl != kEmpty) store(sl, x);
     } else {
         for (u32 i = tid + (R + C::BLOCK - 1) / C::BLOCK * C::NW; i < C::RPT * C::NW; i += C::BLOCK) s_row[i] = 0u;
         scan_rows<C>(s_row, &s_total);
@@ -723,70 +764,87 @@ __device__ __forceinline__ void exec_chunk(const Src &src, const u32 R, const Ba
         if (won >> k & 1u) n_tw += old[k] != stamp;
 }
 
-// A bucket of more than CHUNK records, chunk by chunk: one round over the
-// records finds the distinct cells, reads each once and counts its ops, a
-// second executes, the cells' values carried in shared memory.  The ops on a
-// hot cell are scanned by the whole block, chunk by chunk; the other
-// contended ops are collected, in order, and sorted when the list is full.
-// More distinct cells than the hash holds: class by class of cells.
+// A bucket of more than CHUNK records (a hot cell's), chunk by chunk, the
+// cells' values carried in shared memory and written back at the end.  The
+// next chunk's records are requested before a chunk is executed.  Of a
+// chunk's contended ops those on up to four frequent cells are scanned by the
+// whole block, cell by cell; what is left is compared or sorted.  More
+// distinct cells than the hash holds: class by class of cells, from the
+// start (nothing but outputs, which come out the same, has been written).
+// (Out of line, so that its registers don't spill those of the common case;
+// by value, so that the kernel's parameters need no address.)
 template <class C, class Src>
-__device__ __forceinline__ void exec_long(const Src &src, const u32 R, const BatchDev &b, const Tabs &T,
-                                       const BucketPlan &p, Counters *ctr, const u32 stamp, u32 &n_tw, u32 &n_con,
-                                       u32 &n_m) {
+__device__ __noinline__ void exec_long(const Src src, const u32 R, const BatchDev b, const Tabs &T, const BucketPlan p,
+                                       Counters *ctr, const u32 stamp, u32 *stats) {
+    u32 n_tw = 0, n_con = 0, n_m = 0;
     typedef typename ValT<C::WIDE>::V V;
     typedef typename ValT<C::WIDE>::S S;
-    static_assert(C::HS * 4 <= C::CHUNK * 8, "the counts fit the list's place");
+    static_assert(C::HS * 2 <= C::CHUNK * 4, "16-bit counts fit the ops' place");
     const Smem<C> m;
     u32 *tab = m.tab();
     V *val = m.val();
-    u64 *cl = m.cl(), *stage = m.stage();
-    u32 *count = reinterpret_cast<u32 *>(cl);  // [HS], first round only
-    __shared__ u32 s_distinct, s_nhot, s_hot[kHotCells], s_row[C::RPT * C::NW], s_total;
+    u64 *cl = m.cl();
+    // ops a cell had before it was contended, two 16-bit counts a word (a
+    // longer bucket than 65535 is not executed here)
+    u32 *count = m.op();
+    __shared__ u32 s_distinct, s_con, s_left, s_cand[C::NW], s_row[C::RPT * C::NW], s_total;
     __shared__ S s_sum[C::RPT * C::NW], s_all;
-    const u32 tid = threadIdx.x, chunks = (R + C::CHUNK - 1) / C::CHUNK;
+    const u32 tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     u32 cbits = 0, cval = 0;  // the class of cells executed now: top cbits of their class hash == cval
     auto mine = [&](u32 lc) { return !cbits || ((lc * kClassMul) >> (32 - cbits)) == cval; };
     for (;;) {
         __syncthreads();
-        for (u32 i = tid; i < C::HS; i += C::BLOCK) {
-            tab[i] = kEmpty;
-            count[i] = 0u;
-        }
-        if (tid == 0) s_distinct = s_nhot = 0u;
-        for (u32 c = 0; c < chunks; c++) {
-            const u32 len = min((u32)C::CHUNK, R - c * C::CHUNK);
-            src.template gather_long<C>(c * C::CHUNK, len);
-            __syncthreads();
-            u32 slot[C::RPT], old[C::RPT], won = 0, wide = 0;
+        for (u32 i = tid; i < C::HS; i += C::BLOCK) tab[i] = kEmpty;
+        for (u32 i = tid; i < C::HS / 2; i += C::BLOCK) count[i] = 0u;
+        if (tid == 0) s_distinct = 0u;
+        u64 nx[C::RPT];
+        u32 nt[C::RPT], contended = 0;  // contended: ops executed while their cell was known to be
+        src.template request<C>(0, R, nx, nt);
+        __syncthreads();
+        bool over = false;
+        for (u32 lo = 0; lo < R; lo += C::CHUNK) {
+            Rec r[C::RPT];
+            u32 op[C::RPT], slot[C::RPT], old[C::RPT], in = 0, won = 0, wide = 0;
             V v[C::RPT];
 #pragma unroll
+            for (int k = 0; k < C::RPT; k++)
+                if (lo + (u32)k * C::BLOCK + tid < R) {
+                    r[k] = unpack(nx[k] - ((u64)src.start << 32));
+                    op[k] = nt[k] * src.tile + ((u32)nx[k] & ((1u << kOpBits) - 1u));
+                    if (mine(r[k].lc)) in |= 1u << k;
+                }
+            src.template request<C>(lo + C::CHUNK, R, nx, nt);
+            // ---- new cells, and their values before the batch ----
+            if (tid == 0) s_con = s_left = 0u;
+#pragma unroll
             for (int k = 0; k < C::RPT; k++) {
-                const u32 q = (u32)k * C::BLOCK + tid;
-                bool win = false, in = false;
+                bool win = false, add1 = false;
                 slot[k] = 0;
-                if (q < len && *(volatile u32 *)&s_distinct < C::DISTINCT) {
-                    const Rec r = unpack(stage[q]);
-                    if (mine(r.lc)) {
-                        slot[k] = enter_cell<C>(tab, r.lc, r.add, &win);
-                        in = true;
-                    }
+                if ((in >> k & 1u) && *(volatile u32 *)&s_distinct < C::DISTINCT) {
+                    slot[k] = enter_cell<C>(tab, r[k].lc, r[k].add, &win);
                     if (win) {
                         bool wd;
-                        const u32 cell = src.cell(r.lc);
+                        const u32 cell = src.cell(r[k].lc);
                         const char *a = cell_addr(T, cell, &wd);
                         v[k] = (V)load_cell(a, C::WIDE && wd);
                         old[k] = atomicExch(&p.epoch[cell >> p.word_shift], stamp);
                         won |= 1u << k;
                         if (C::WIDE && wd) wide |= 1u << k;
                     }
+                    if (is_contended(tab[slot[k]])) contended++;
+                    else add1 = true;
                 }
-                // the first op's cell is counted for the whole warp: likely the hot one
-                const u32 ins = __ballot_sync(FULL_MASK, in);
-                const int ld = ins ? __ffs(ins) - 1 : 0;
-                const u32 first = __shfl_sync(FULL_MASK, slot[k], ld);
-                const u32 peers = __ballot_sync(FULL_MASK, in && slot[k] == first);
-                if (in && (!(peers >> lane & 1u) || lane == ld)) atomicAdd(&count[slot[k]], lane == ld ? (u32)__popc(peers) : 1u);
+                // an op on a cell not yet contended is counted there; the
+                // first such op's cell for the whole warp
+                const u32 some = __ballot_sync(FULL_MASK, add1);
+                if (some) {
+                    const int ld = __ffs(some) - 1;
+                    const u32 first = __shfl_sync(FULL_MASK, slot[k], ld);
+                    const u32 peers = __ballot_sync(FULL_MASK, add1 && slot[k] == first);
+                    if (add1 && (lane == ld || !(peers >> lane & 1u)))
+                        atomicAdd(&count[slot[k] >> 1], (lane == ld ? (u32)__popc(peers) : 1u) << (16 * (slot[k] & 1u)));
+                }
                 const u32 bal = __ballot_sync(FULL_MASK, win);
                 if (lane == 0 && bal) atomicAdd(&s_distinct, (u32)__popc(bal));
             }
@@ -798,103 +856,127 @@ __device__ __forceinline__ void exec_long(const Src &src, const u32 R, const Bat
                     n_tw += old[k] != stamp;
                 }
             __syncthreads();
+            if (s_distinct >= C::DISTINCT) {  // too many
+                over = true;
+                break;
+            }
+            // ---- ops on cells without a conflict so far; the others counted ----
+            u32 con = 0, wd = 0, cand = kEmpty;
+            V base[C::RPT];
+#pragma unroll
+            for (int k = 0; k < C::RPT; k++)
+                if (in >> k & 1u) {
+                    const u32 t = tab[slot[k]];
+                    base[k] = val[slot[k]];
+                    if (C::WIDE && (t & kWideCell)) wd |= 1u << k;
+                    if (is_contended(t)) {
+                        con |= 1u << k;
+                        cand = slot[k];
+                    } else {
+                        V y = base[k];
+                        if (r[k].add) {  // its first op
+                            y = narrow<C>((V)((S)y + (S)(V)r[k].imm), t & kWideCell);
+                            val[slot[k]] = y;
+                        }
+                        put_out<C>(b, ctr, op[k], y, t & kWideCell);
+                    }
+                }
+            {
+                const u32 c = __reduce_add_sync(FULL_MASK, (u32)__popc(con));
+                const u32 some = __ballot_sync(FULL_MASK, con != 0u);
+                cand = __shfl_sync(FULL_MASK, cand, some ? __ffs(some) - 1 : 0);
+                if (lane == 0) {
+                    if (c) atomicAdd(&s_con, c);
+                    s_cand[warp] = cand;
+                }
+            }
+            __syncthreads();
+            u32 left = s_con;
+            // ---- frequent cells: an ordered scan each ----
+#pragma unroll 1
+            for (int h = 0; h < kHotTries && left > kFew; h++) {
+                const u32 sl = s_cand[h * (C::NW / kHotTries)];
+                bool seen = sl == kEmpty;
+                for (int j = 0; j < h; j++) seen = seen || s_cand[j * (C::NW / kHotTries)] == sl;
+                if (seen) continue;  // the same for the block
+                S sum[C::RPT];
+                u32 on = 0, rank[C::RPT];
+#pragma unroll
+                for (int k = 0; k < C::RPT; k++) {
+                    const bool x = (con >> k & 1u) && slot[k] == sl;
+                    if (x) on |= 1u << k;
+                    sum[k] = x ? (S)(V)r[k].imm : (S)0;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const S y = __shfl_up_sync(FULL_MASK, sum[k], d);
+                        if (lane >= d) sum[k] += y;
+                    }
+                    const u32 bal = __ballot_sync(FULL_MASK, x);
+                    rank[k] = (u32)__popc(bal & lanemask_lt());
+                    if (lane == 31) {
+                        s_sum[k * C::NW + warp] = sum[k];
+                        s_row[k * C::NW + warp] = (u32)__popc(bal);
+                    }
+                }
+                scan_rows<C>(s_sum, &s_all);
+                const u32 total = scan_rows<C>(s_row, &s_total);
+#pragma unroll
+                for (int k = 0; k < C::RPT; k++)
+                    if (on >> k & 1u) {
+                        const V y = narrow<C>((V)((S)base[k] + s_sum[k * C::NW + warp] + sum[k]), wd >> k & 1u);
+                        put_out<C>(b, ctr, op[k], y, wd >> k & 1u);
+                        if (s_row[k * C::NW + warp] + rank[k] + 1u == total) val[sl] = y;
+                    }
+                con &= ~on;
+                left -= total;
+                __syncthreads();
+            }
+            if (left > kFew) {
+#pragma unroll
+                for (int k = 0; k < C::RPT; k++) {
+                    const u32 bal = __ballot_sync(FULL_MASK, con >> k & 1u);
+                    if (lane == 0) s_row[k * C::NW + warp] = (u32)__popc(bal);
+                }
+                scan_rows<C>(s_row, &s_total);
+#pragma unroll
+                for (int k = 0; k < C::RPT; k++) {
+                    const bool cn = con >> k & 1u;
+                    const u32 bal = __ballot_sync(FULL_MASK, cn);
+                    if (cn) cl[s_row[k * C::NW + warp] + __popc(bal & lanemask_lt())] = entry(slot[k], r[k].imm, op[k]);
+                }
+                run_sorted<C>(m, left, b, ctr, [&](u32 sl, V y) { val[sl] = y; });
+            } else if (left) {
+#pragma unroll
+                for (int k = 0; k < C::RPT; k++) {
+                    const bool cn = con >> k & 1u;
+                    const u32 bal = __ballot_sync(FULL_MASK, cn);
+                    if (!bal) continue;
+                    u32 at = 0;
+                    if (lane == 0) at = atomicAdd(&s_left, (u32)__popc(bal));
+                    at = __shfl_sync(FULL_MASK, at, 0) + (u32)__popc(bal & lanemask_lt());
+                    if (cn) cl[at] = entry(slot[k], r[k].imm, op[k]);
+                }
+                __syncthreads();
+                V y = 0;
+                const u32 sl = compare_all<C>(m, left, b, ctr, &y);
+                __syncthreads();
+                if (sl != kEmpty) val[sl] = y;
+            }
+            __syncthreads();
         }
-        if (s_distinct >= C::DISTINCT) {  // too many: half the class
+        if (over) {  // half the class
             cbits++;
             cval <<= 1;
             continue;
         }
-        for (u32 i = tid; i < C::HS; i += C::BLOCK)
-            if (tab[i] != kEmpty && is_contended(tab[i]) && count[i] > kHot) {
-                const u32 h = atomicAdd(&s_nhot, 1u);
-                if (h < kHotCells) s_hot[h] = i;
-            }
-        __syncthreads();
-        const u32 n_hot = min(s_nhot, kHotCells);
-        u32 listed = 0;  // contended ops in cl
-        for (u32 c = 0; c < chunks; c++) {
-            const u32 len = min((u32)C::CHUNK, R - c * C::CHUNK);
-            src.template gather_long<C>(c * C::CHUNK, len);
-            __syncthreads();
-            u64 x[C::RPT];  // entries of this thread's contended ops
-            u32 con = 0, which = 0;  // which: hot cell + 1, four bits a row
-#pragma unroll
-            for (int k = 0; k < C::RPT; k++) {
-                const u32 q = (u32)k * C::BLOCK + tid;
-                x[k] = 0ull;
-                if (q >= len) continue;
-                const Rec r = unpack(stage[q]);
-                if (!mine(r.lc)) continue;
-                u32 sl = (r.lc * kSlotMul) >> (32 - C::HB);
-                while ((tab[sl] >> 3) != r.lc) sl = (sl + 1) & (C::HS - 1);
-                const u32 t = tab[sl], op = src.op(q);
-                if (is_contended(t)) {
-                    n_con++;
-                    x[k] = entry(sl, r.imm, op);
-                    u32 h = 0;
-                    for (u32 j = 0; j < n_hot; j++)
-                        if (s_hot[j] == sl) h = j + 1u;
-                    if (h) which |= h << (4 * k);
-                    else con |= 1u << k;
-                    continue;
-                }
-                V y = val[sl];
-                if (r.add) {
-                    y = narrow<C>((V)((S)y + (S)(V)r.imm), t & kWideCell);
-                    val[sl] = y;
-                }
-                put_out<C>(b, ctr, op, y, t & kWideCell);
-            }
-#pragma unroll 1
-            for (u32 h = 0; h < n_hot; h++) {
-                const u32 sl = s_hot[h];
-                const bool wd = C::WIDE && (tab[sl] & kWideCell);
-                S in[C::RPT];
-#pragma unroll
-                for (int k = 0; k < C::RPT; k++) {
-                    in[k] = (which >> (4 * k) & 15u) == h + 1u ? (S)(V)imm20((u32)(x[k] >> 32)) : (S)0;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const S y = __shfl_up_sync(FULL_MASK, in[k], d);
-                        if (lane >= d) in[k] += y;
-                    }
-                    if (lane == 31) s_sum[k * C::NW + warp] = in[k];
-                }
-                const S all = scan_rows<C>(s_sum, &s_all), base = (S)val[sl];
-#pragma unroll
-                for (int k = 0; k < C::RPT; k++)
-                    if ((which >> (4 * k) & 15u) == h + 1u)
-                        put_out<C>(b, ctr, (u32)x[k], narrow<C>((V)(base + s_sum[k * C::NW + warp] + in[k]), wd), wd);
-                __syncthreads();
-                if (tid == 0) val[sl] = narrow<C>((V)(base + all), wd);
-                __syncthreads();
-            }
-#pragma unroll
-            for (int k = 0; k < C::RPT; k++) {
-                const u32 bal = __ballot_sync(FULL_MASK, con >> k & 1u);
-                if (lane == 0) s_row[k * C::NW + warp] = (u32)__popc(bal);
-            }
-            const u32 more = scan_rows<C>(s_row, &s_total);
-            if (listed + more > C::CHUNK) {
-                run_sorted<C>(m, listed, b, ctr, [&](u32 sl, V y) { val[sl] = y; });
-                listed = 0;
-                __syncthreads();
-            }
-#pragma unroll
-            for (int k = 0; k < C::RPT; k++) {
-                const bool cn = con >> k & 1u;
-                const u32 bal = __ballot_sync(FULL_MASK, cn);
-                if (cn) cl[listed + s_row[k * C::NW + warp] + __popc(bal & lanemask_lt())] = x[k];
-            }
-            listed += more;
-            __syncthreads();
-        }
-        if (listed) run_sorted<C>(m, listed, b, ctr, [&](u32 sl, V y) { val[sl] = y; });
-        __syncthreads();
+        n_con += contended;
         for (u32 i = tid; i < C::HS; i += C::BLOCK) {
             const u32 t = tab[i];
             if (t == kEmpty) continue;
-            n_m += is_contended(t);
+            if (is_contended(t)) {
+                n_m++;
+                n_con += count[i >> 1] >> (16 * (i & 1u)) & 0xFFFFu;
+            }
             if (t & kWritten) {
                 bool wd;
                 char *a = cell_addr(T, src.cell(t >> 3), &wd);
@@ -909,15 +991,19 @@ __device__ __forceinline__ void exec_long(const Src &src, const u32 R, const Bat
         }
         if (!cbits) break;
     }
+    stats[0] = n_tw;
+    stats[1] = n_con;
+    stats[2] = n_m;
 }
 
 // Records of one bucket, tile by tile.
 struct TileSrc {
     const u64 *recs;
-    const uint16_t *offs;  // the bucket's column
     u32 *ops;              // ops of the staged records (shared memory)
-    const u32 *pre;        // long buckets: records of the bucket before each tile (shared memory)
-    u32 stride, n_tiles, tile;
+    // long buckets (shared memory): records of the bucket before each tile,
+    // and where its first one lies minus that
+    const u32 *pre, *adj;
+    u32 n_tiles, tile;
     u32 cell_bits, start;  // start: first mixed cell number of the bucket
     __device__ __forceinline__ u32 cell(u32 lc) const { return unmix_cell(start + lc, cell_bits); }
     __device__ __forceinline__ u32 op(u32 q) const { return ops[q]; }
@@ -925,19 +1011,24 @@ struct TileSrc {
         stage[q] = x - ((u64)start << 32);
         ops[q] = t * tile + ((u32)x & ((1u << kOpBits) - 1u));
     }
-    // records [lo, lo + len) of a long bucket: each looks its tile up
+    // Requests record lo + q of a long bucket for q = k * BLOCK + thread
+    // (below R in all); t: their tiles.  The warp finds its first record's
+    // tile with two rounds of 32 comparisons, each lane walks on from there.
     template <class C>
-    __device__ __forceinline__ void gather_long(u32 lo, u32 len) const {
-        u64 *stage = Smem<C>().stage();
-        const u32 top = 1u << (31 - __clz((int)n_tiles));
+    __device__ __forceinline__ void request(u32 lo, u32 R, u64 (&x)[C::RPT], u32 (&t)[C::RPT]) const {
+        const u32 lane = threadIdx.x & 31;
 #pragma unroll
         for (int k = 0; k < C::RPT; k++) {
-            const u32 q = (u32)k * C::BLOCK + threadIdx.x, pos = lo + q;
-            if (q >= len) continue;
-            u32 t = 0;  // the last tile with pre[t] <= pos
-            for (u32 s = top; s; s >>= 1)
-                if (t + s < n_tiles && pre[t + s] <= pos) t += s;
-            put(stage, q, __ldcs(&recs[(u64)t * tile + offs[(u64)t * stride] + (pos - pre[t])]), t);
+            const u32 pos = lo + (u32)k * C::BLOCK + threadIdx.x, first = pos - lane;
+            if (first >= R) break;  // the same for the warp
+            const u32 g = (u32)__popc(__ballot_sync(FULL_MASK, lane * 32 < n_tiles && pre[lane * 32] <= first)) - 1u;
+            const u32 i = g * 32 + lane;
+            u32 at = g * 32 + (u32)__popc(__ballot_sync(FULL_MASK, i < n_tiles && pre[i] <= first)) - 1u;
+            if (pos < R) {
+                while (at + 1 < n_tiles && pre[at + 1] <= pos) at++;
+                t[k] = at;
+                x[k] = __ldcs(&recs[adj[at] + pos]);
+            }
         }
     }
 };
@@ -1050,13 +1141,13 @@ __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T,
     const bool extra = blockIdx.x == p.n_buckets;  // with inserts: one block more
     TileSrc src;
     src.recs = p.recs;
-    src.stride = p.n_buckets + 1;
-    src.offs = p.offs + blockIdx.x;
+    const uint16_t *offs = p.offs + blockIdx.x;  // the bucket's column
     src.ops = Smem<C>().op();
     src.pre = Smem<C>().pre();
+    src.adj = Smem<C>().adj();
     src.n_tiles = p.n_tiles;
     src.tile = p.tile;
-    const u32 per = p.n_tiles > (u32)C::BLOCK ? TPT : 1;
+    const u32 per = (p.n_tiles + C::BLOCK - 1) / C::BLOCK;
     u32 at[TPT], cnt[TPT], len = 0, R;
     u64 x[TPT][PRE];
 #pragma unroll
@@ -1064,7 +1155,7 @@ __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T,
         const u32 t = tid * per + (u32)j;
         at[j] = cnt[j] = 0;
         if (!extra && (u32)j < per && t < p.n_tiles) {
-            const uint16_t *o = src.offs + (u64)t * src.stride;
+            const uint16_t *o = offs + (u64)t * (p.n_buckets + 1);
             at[j] = o[0];
             cnt[j] = o[1] - at[j];
         }
@@ -1116,14 +1207,21 @@ __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T,
         src.cell_bits = p.cell_bits;
         src.start = blockIdx.x * p.width;
         if (R > C::CHUNK) {
-            u32 *pre = Smem<C>().pre();
+            u32 *pre = Smem<C>().pre(), *adj = Smem<C>().adj();
 #pragma unroll
-            for (int j = 0; j < TPT; j++)
-                if ((u32)j < per && tid * per + (u32)j < p.n_tiles) {
-                    pre[tid * per + (u32)j] = pos;
+            for (int j = 0; j < TPT; j++) {
+                const u32 t = tid * per + (u32)j;
+                if ((u32)j < per && t < p.n_tiles) {
+                    pre[t] = pos;
+                    adj[t] = t * p.tile + at[j] - pos;
                     pos += cnt[j];
                 }
-            exec_long<C>(src, R, b, s_tabs, p, p.snap, stamp, n_tw, n_con, n_m);
+            }
+            u32 stats[3];
+            exec_long<C>(src, R, b, s_tabs, p, p.snap, stamp, stats);
+            n_tw = stats[0];
+            n_con = stats[1];
+            n_m = stats[2];
         } else if (R) {
             u64 *stage = Smem<C>().stage();
 #pragma unroll
@@ -1298,7 +1396,7 @@ cudaError_t go_part(const Launch &L, const BatchDev &b, const TablesDev &T, cons
 
 constexpr u64 kSoloSmall = 1024, kSoloOps = 2048;  // batches that one block executes
 constexpr u64 kPartOps = 2ull << 20;               // largest batch that is split
-constexpr u32 kBucketLimit = 32768;                // a longer bucket would keep one block busy for too long
+constexpr u32 kBucketLimit = 32767;                // a longer bucket would keep one block busy for too long
 constexpr u32 kMaxLcBits = 28;                     // the slot word holds a cell number and three flags
 
 // Can the batch go this way, and how is it split?
@@ -1321,11 +1419,12 @@ bool plan_buckets(const Launch &L, const BatchDev &b, const TablesDev &T, const 
     p->word_shift = L.tune.word_bits == 64 && tiling_supported((int)L.tune.block, (int)L.tune.ipt, 64) ? 6 : 5;
     *solo = n <= kSoloOps && cb <= kMaxLcBits;
     if (*solo) return true;
-    // whole waves of two blocks per SM once the buckets are full enough,
-    // fewer and smaller buckets before that
+    // Whole waves of two blocks per SM, their buckets well inside a chunk: a
+    // small batch is spread over all of them too (65,536 Zipf ops a batch,
+    // the request log: 304 buckets 550 us a pass, 128 buckets 575; 12 uneven
+    // batches of 17,000 to 270,000 ops: 226 and 246 us)
     const u32 wave = 2u * (u32)L.num_sms;
-    u32 nb = n / 512 < wave ? n / 512 : wave * ((n + wave * 1700 - 1) / (wave * 1700));
-    if (nb < 16) nb = 16;
+    u32 nb = wave * ((n + wave * 1700 - 1) / (wave * 1700));
     if (cb > kMaxLcBits && nb < 1u << (cb - kMaxLcBits)) nb = 1u << (cb - kMaxLcBits);
     if (nb > 1u << (cb - 1)) nb = 1u << (cb - 1);
     p->width = (u32)(((1ull << cb) + nb - 1) / nb);
