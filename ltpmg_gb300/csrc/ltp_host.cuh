@@ -45,6 +45,7 @@ struct ltp_ctx {
     std::string last_error;
     Tuning tuning[64];
     uint32_t stall_ms_next = 0;
+    uint8_t *h_stage = nullptr;  // pinned staging of synchronous results (null: copied straight)
     bool dirty = false;  // scratch must be reset before the next batch
     // multi-batch execution: cached CUDA graph and persistent-kernel buffers
     std::vector<uint64_t> graph_key;
@@ -66,6 +67,7 @@ struct ltp_batch {
     uint32_t *keys32 = nullptr;  // 32-bit keys (allocated at the first ltp_batch_load32)
     bool key32 = false;          // the loaded batch carries 32-bit keys
     uint32_t *opw = nullptr, *txn_first = nullptr, *op_txn = nullptr;
+    uint8_t *results = nullptr;  // one allocation: snap, commit and out
     int32_t *out = nullptr;
     long long *out64 = nullptr;  // full outputs, allocated once the context has int64 columns
     uint8_t *commit = nullptr;

@@ -134,6 +134,7 @@ def load():
         "ltp_batch_fetch64": (ci, [vp, vp, vp, vp]),
         "ltp_batch_finish": (ci, [vp, vp, ctypes.POINTER(Stats), vp]),
         "ltp_batch_results": (ci, [vp, vp, vp, vp, ctypes.POINTER(Stats)]),
+        "ltp_batch_results64": (ci, [vp, vp, vp, vp, ctypes.POINTER(Stats)]),
         "ltp_batch_device_ptrs": (ci, [vp, pp, pp, pp, pp, pp]),
         "ltp_host_alloc": (vp, [ctypes.c_size_t]),
         "ltp_host_free": (None, [vp]),
@@ -538,19 +539,18 @@ class Batch:
         return st
 
     def results(self):
-        commit = np.zeros(max(self.n_txns, 1), np.uint8)
-        vals = np.zeros(max(self.n_ops, 1), np.int32)
+        commit = np.empty(max(self.n_txns, 1), np.uint8)
+        vals = np.empty(max(self.n_ops, 1), np.int32)
         st = Stats()
         self.ctx.check(self.ctx.L.ltp_batch_results(self.ctx.h, self.h, _p(commit), _p(vals), ctypes.byref(st)))
         return commit[: self.n_txns], vals[: self.n_ops], st
 
     def results64(self):
         """(commit, int64 values, stats); the context must have an int64 column."""
-        commit = np.zeros(max(self.n_txns, 1), np.uint8)
-        vals = np.zeros(max(self.n_ops, 1), np.int64)
-        self.fetch(commit=commit)
-        self.fetch64(vals)
-        st = self.finish()
+        commit = np.empty(max(self.n_txns, 1), np.uint8)
+        vals = np.empty(max(self.n_ops, 1), np.int64)
+        st = Stats()
+        self.ctx.check(self.ctx.L.ltp_batch_results64(self.ctx.h, self.h, _p(commit), _p(vals), ctypes.byref(st)))
         return commit[: self.n_txns], vals[: self.n_ops], st
 
 
