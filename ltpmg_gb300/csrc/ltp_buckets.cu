@@ -189,8 +189,12 @@ size_t part_smem(u32 tile, u32 buckets) {
     return (size_t)tile * 8 + (size_t)(kPartBlock / 32) * ((buckets + 1) / 2) * 4;
 }
 
+// Two blocks per SM, not three: a tile's ops are held in registers from their
+// loads to the records, and at the 40 registers that three blocks leave they
+// spill (order entry 468 -> 461 us, 32,768 x 55 read-only ops 164 -> 161 us,
+// 65,536 x 10 with snapshots 173 -> 170 us).
 template <int IPT>
-__global__ void __launch_bounds__(kPartBlock, 3) k_part(BatchDev b, TablesDev T, BucketPlan p) {
+__global__ void __launch_bounds__(kPartBlock, 2) k_part(BatchDev b, TablesDev T, BucketPlan p) {
     pdl_begin();
     constexpr int NW = kPartBlock / 32;
     constexpr u32 TILE = kPartBlock * IPT;
