@@ -2065,7 +2065,10 @@ constexpr size_t kPersistSmem = 4ull * 2 * kPBlock * kPIpt * sizeof(u32) > kInsS
 
 __global__ void __launch_bounds__(kPBlock, 2) k_persist(PersistArgs a) {
     const u32 nb = gridDim.x;
-    if (a.gate && !*(volatile u32 *)&a.gate->skew) return;
+    if (a.gate) {
+        pdl_begin();
+        if (!*(volatile u32 *)&a.gate->skew) return;
+    }
     for (u32 j = 0; j < a.n_batches; j++) {
         const BatchDev b = a.gate ? a.one : a.batches[j];
         if (a.gate && b.payload_len) {  // the bucket path counted the inserts
@@ -2174,8 +2177,22 @@ cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev 
     a.gate = s.pstate;
     a.one = b;
     a.one_snap = snap;
-    void *args[] = {&a};
-    return cudaLaunchCooperativeKernel((const void *)k_persist, dim3(grid), dim3(kPBlock), args, kPersistSmem, L.stream);
+    // Cooperative, and by dependent launch: nearly always it only looks at the
+    // gate, and its launch then hides behind the bucket kernel (six batches of
+    // 327,680 ops 311 -> 307 us, 65536 x 10 with snapshots 174 -> 170 us).
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(kPBlock);
+    c.dynamicSmemBytes = kPersistSmem;
+    c.stream = L.stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 2;
+    return cudaLaunchKernelEx(&c, k_persist, a);
 }
 
 int persistent_grid(int num_sms) {
