@@ -384,6 +384,8 @@ __device__ __forceinline__ u64 entry(u32 slot, int imm, u32 op) {
     return ((u64)(slot << 20 | ((u32)imm & 0xFFFFFu)) << 32) | op;
 }
 
+constexpr u32 kClassSlots = 8;  // neighbouring slots whose contended ops are compared with one another
+
 template <int BLOCK_, int RPT_, int HB_, bool WIDE_>
 struct Cfg {
     static constexpr int BLOCK = BLOCK_, RPT = RPT_, HB = HB_, NW = BLOCK / 32;
@@ -394,6 +396,8 @@ struct Cfg {
     // insertions stop here: each thread may add one more before it sees the
     // count, and the probe loops need an empty slot to end on
     static constexpr u32 DISTINCT = HS - HS / 4;
+    static constexpr u32 NC = HS / kClassSlots;  // classes of contended ops
+    static_assert(NC <= (u32)BLOCK && NC < NW * ND, "a thread looks after a class");
     static_assert(DISTINCT + BLOCK <= HS && CHUNK < HS && ND <= (u32)BLOCK && NW <= 32 && RPT * NW <= 64 && HB == 12,
                   "layout");
     static constexpr u32 VB = WIDE ? 8 : 4;
@@ -413,8 +417,9 @@ struct ValT<true> {
 };
 
 constexpr u32 kEmpty = 0xFFFFFFFFu;
-constexpr u32 kFew = 256;  // contended ops of a chunk that are resolved all against all
-constexpr int kHotTries = 4;  // cells of a chunk with more that are scanned for themselves
+constexpr u32 kFew = 256;       // as many at most: the comparisons grow with the square
+constexpr u32 kTiny = 64;       // so few in all are compared without classes
+constexpr int kHotTries = 4;    // frequent cells of a long bucket's chunk that are scanned for themselves
 // slot word: cell number << 3 | these
 constexpr u32 kWritten = 1u, kMulti = 2u, kWideCell = 4u;
 
@@ -630,32 +635,74 @@ __device__ __forceinline__ void run_sorted(const Smem<C> &m, const u32 rc, const
     }
 }
 
-// Executes rc <= kFew contended ops that cl holds in any order: each looks
-// at all of them, its cell's value is the sum over the ops on it up to its
-// own.  Returns the slot, and in *x the last value, of a cell whose last op is
-// this thread's, else kEmpty.
+// The classes' counts (cnt, each op counted by its slot) become their first
+// places; false if some class has more than kFew.
 template <class C>
-__device__ __forceinline__ u32 compare_all(const Smem<C> &m, const u32 rc, const BatchDev &b, Counters *ctr,
-                                           typename ValT<C::WIDE>::V *x) {
+__device__ __forceinline__ bool class_starts(const Smem<C> &m) {
+    __shared__ u32 s_wc[C::NW], s_big;
+    const u32 tid = threadIdx.x;
+    u32 *cnt = m.cnt(), rc;
+    const u32 c = tid < C::NC ? cnt[tid] : 0u;
+    if (tid == 0) s_big = 0u;
+    const u32 off = block_excl<C::NW>(c, s_wc, &rc);
+    if (c > kFew) s_big = 1u;
+    if (tid < C::NC) cnt[tid] = off;
+    if (tid == 0) cnt[C::NC] = rc;
+    __syncthreads();
+    return s_big == 0u;
+}
+
+// Executes the rc contended ops that cl holds class by class, in any order
+// inside a class (WHOLE: in any order): each looks at its class, its cell's value is the sum over
+// the ops on it up to its own.  done(slot, value) for the last op of every
+// cell, AFTER: once every value has been read.
+//
+// Bound by instruction issue: all of a chunk's ops against all took a third of
+// a block's time on order entry (250 ops: 13,000 cycles), by classes of eight
+// slots an op meets a handful of others (order entry 461 -> 437 us, six
+// batches of 327,680 ops in the pipeline 307 -> 276, 1.5 M uniform ops 92 ->
+// 74; classes of sixteen the same).  The classes' scan costs two barriers: up
+// to kTiny ops do without (3,000 ops 9.7 -> 9.2 us, uneven batches 207 -> 201
+// us; 16 and 32: 207 and 204).
+template <class C, bool AFTER, bool WHOLE, class Done>
+__device__ __forceinline__ void compare(const Smem<C> &m, const u32 rc, const BatchDev &b, Counters *ctr, Done done) {
     typedef typename ValT<C::WIDE>::V V;
     typedef typename ValT<C::WIDE>::S S;
-    if (threadIdx.x >= rc) return kEmpty;
     const u64 *cl = m.cl();
-    const u64 me = cl[threadIdx.x];
-    const u32 sl = (u32)(me >> 52), op = (u32)me;
-    u32 later = 0;
-    S sum = 0;
-#pragma unroll 8
-    for (u32 j = 0; j < rc; j++) {
-        const u64 o = cl[j];
-        const bool same = (u32)(o >> 52) == sl, upto = (u32)o <= op;
-        sum += same && upto ? (S)(V)imm20((u32)(o >> 32)) : (S)0;
-        later |= same && !upto;
+    const u32 *cnt = m.cnt();
+    V x[C::RPT];
+    u32 last[C::RPT];
+#pragma unroll
+    for (int k = 0; k < C::RPT; k++) {
+        const u32 q = (u32)k * C::BLOCK + threadIdx.x;
+        last[k] = kEmpty;
+        if (q >= rc) continue;
+        const u64 me = cl[q];
+        const u32 hi = (u32)(me >> 32) & 0xFFF00000u, sl = (u32)(me >> 52), op = (u32)me;
+        const u32 to = WHOLE ? rc : cnt[sl / kClassSlots + 1];  // (of the last class: rc)
+        bool later = false;
+        int sum = 0;  // (256 increments of 20 bits)
+#pragma unroll 4
+        for (u32 j = WHOLE ? 0u : cnt[sl / kClassSlots]; j < to; j++) {
+            const u64 o = cl[j];
+            const u32 d = (u32)(o >> 32) - hi;  // same slot: the increment
+            const bool same = d < 1u << 20, upto = (u32)o <= op;
+            sum += same && upto ? imm20(d) : 0;
+            later = later || (same && !upto);
+        }
+        const bool wd = C::WIDE && (m.tab()[sl] & kWideCell);
+        x[k] = narrow<C>((V)((S)m.val()[sl] + (S)(V)sum), wd);
+        put_out<C>(b, ctr, op, x[k], wd);
+        if (later) continue;
+        if (AFTER) last[k] = sl;
+        else done(sl, x[k]);
     }
-    const bool wd = C::WIDE && (m.tab()[sl] & kWideCell);
-    *x = narrow<C>((V)((S)m.val()[sl] + sum), wd);
-    put_out<C>(b, ctr, op, *x, wd);
-    return later ? kEmpty : sl;
+    if (AFTER) {
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < C::RPT; k++)
+            if (last[k] != kEmpty) done(last[k], x[k]);
+    }
 }
 
 // Executes the R <= CHUNK records that are staged (op order; kNoRec: none).
@@ -671,11 +718,13 @@ __device__ __forceinline__ void exec_chunk(const Src &src, const u32 R, const Ba
     V *val = m.val();
     u64 *cl = m.cl();
     const u64 *stage = m.stage();
-    __shared__ u32 s_con, s_row[C::RPT * C::NW], s_total;
+    u32 *cnt = m.cnt();
+    __shared__ u32 s_con, s_at, s_row[C::RPT * C::NW], s_total;
     const u32 tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
+    if (tid < C::NC) cnt[tid] = 0u;
+    if (tid == 0) s_con = s_at = 0u;
     for (u32 i = tid; i < C::HS / 4; i += C::BLOCK) reinterpret_cast<uint4 *>(tab)[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
-    if (tid == 0) s_con = 0u;
     __syncthreads();
     // every op reads its cell while the hash is built: the value before the
     // batch, which is what all but the contended ops need
@@ -709,36 +758,29 @@ __device__ __forceinline__ void exec_chunk(const Src &src, const u32 R, const Ba
     for (int k = 0; k < C::RPT; k++) {
         if ((u32)k * C::BLOCK >= R) break;
         const u32 q = (u32)k * C::BLOCK + tid;
-        bool cn = false;
-        Rec r;
-        if (has >> k & 1u) {
-            r = unpack(stage[q]);
-            const bool wd = C::WIDE && (wide >> k & 1u);
-            cn = is_contended(tab[slot[k]]);
-            if (!cn) {  // the cell's only op, or one of its reads
-                V x = v[k];
-                if (r.add) {
-                    x = narrow<C>((V)((S)x + (S)(V)r.imm), wd);
-                    store_cell(ptr[k], wd, (long long)x);
-                }
-                put_out<C>(b, ctr, src.op(q), x, wd);
-            } else if (won >> k & 1u) {
+        if (!(has >> k & 1u)) continue;
+        const Rec r = unpack(stage[q]);
+        const bool wd = C::WIDE && (wide >> k & 1u);
+        if (!is_contended(tab[slot[k]])) {  // the cell's only op, or one of its reads
+            V x = v[k];
+            if (r.add) {
+                x = narrow<C>((V)((S)x + (S)(V)r.imm), wd);
+                store_cell(ptr[k], wd, (long long)x);
+            }
+            put_out<C>(b, ctr, src.op(q), x, wd);
+        } else {
+            con |= 1u << k;
+            if (won >> k & 1u) {
                 val[slot[k]] = v[k];
                 if (C::WIDE && wd) atomicOr(&tab[slot[k]], kWideCell);
                 n_m++;
             }
-        }
-        if (cn) con |= 1u << k;
-        const u32 bal = __ballot_sync(FULL_MASK, cn);
-        if (lane == 0) s_row[k * C::NW + warp] = (u32)__popc(bal);
-        if (bal) {  // listed in any order: few are compared by op, many are listed again
-            u32 at = 0;
-            if (lane == 0) at = atomicAdd(&s_con, (u32)__popc(bal));
-            at = __shfl_sync(FULL_MASK, at, 0) + (u32)__popc(bal & lanemask_lt());
-            if (cn && at < kFew) cl[at] = entry(slot[k], r.imm, src.op(q));
+            slot[k] |= atomicAdd(&cnt[slot[k] / kClassSlots], 1u) << C::HB;  // its rank in its class
         }
     }
     n_con += (u32)__popc(con);
+    const u32 some = __reduce_add_sync(FULL_MASK, (u32)__popc(con));
+    if (lane == 0 && some) atomicAdd(&s_con, some);
     __syncthreads();
     const u32 rc = s_con;
     auto store = [&](u32 sl, V x) {  // a contended cell's last value
@@ -746,20 +788,35 @@ __device__ __forceinline__ void exec_chunk(const Src &src, const u32 R, const Ba
         char *a = cell_addr(T, src.cell(tab[sl] >> 3), &wd);
         store_cell(a, wd, (long long)x);
     };
+    auto ent = [&](int k) {
+        const u32 q = (u32)k * C::BLOCK + tid;
+        return entry(slot[k] & (C::HS - 1), unpack(stage[q]).imm, src.op(q));
+    };
     if (rc == 0) {
-    } else if (rc <= kFew) {
-        V x = 0;
-        const u32 sl = compare_all<C>(m, rc, b, ctr, &x);
-        if (sl != kEmpty) store(sl, x);
+    } else if (rc <= kTiny) {
+#pragma unroll
+        for (int k = 0; k < C::RPT; k++)
+            if (con >> k & 1u) cl[atomicAdd(&s_at, 1u)] = ent(k);
+        __syncthreads();
+        compare<C, false, true>(m, rc, b, ctr, store);
+    } else if (class_starts<C>(m)) {
+#pragma unroll
+        for (int k = 0; k < C::RPT; k++)
+            if (con >> k & 1u) cl[cnt[(slot[k] & (C::HS - 1)) / kClassSlots] + (slot[k] >> C::HB)] = ent(k);
+        __syncthreads();
+        compare<C, false, false>(m, rc, b, ctr, store);
     } else {
-        for (u32 i = tid + (R + C::BLOCK - 1) / C::BLOCK * C::NW; i < C::RPT * C::NW; i += C::BLOCK) s_row[i] = 0u;
+#pragma unroll
+        for (int k = 0; k < C::RPT; k++) {
+            const u32 bal = __ballot_sync(FULL_MASK, con >> k & 1u);
+            if (lane == 0) s_row[k * C::NW + warp] = (u32)__popc(bal);
+        }
         scan_rows<C>(s_row, &s_total);
 #pragma unroll
         for (int k = 0; k < C::RPT; k++) {
-            const u32 q = (u32)k * C::BLOCK + tid;
             const bool cn = con >> k & 1u;
             const u32 bal = __ballot_sync(FULL_MASK, cn);
-            if (cn) cl[s_row[k * C::NW + warp] + __popc(bal & lanemask_lt())] = entry(slot[k], unpack(stage[q]).imm, src.op(q));
+            if (cn) cl[s_row[k * C::NW + warp] + __popc(bal & lanemask_lt())] = ent(k);
         }
         run_sorted<C>(m, rc, b, ctr, store);
     }
@@ -771,8 +828,9 @@ __device__ __forceinline__ void exec_chunk(const Src &src, const u32 R, const Ba
 // A bucket of more than CHUNK records (a hot cell's), chunk by chunk, the
 // cells' values carried in shared memory and written back at the end.  The
 // next chunk's records are requested before a chunk is executed.  Of a
-// chunk's contended ops those on up to four frequent cells are scanned by the
-// whole block, cell by cell; what is left is compared or sorted.  More
+// chunk's contended ops those on up to four cells that are frequent inside a
+// warp are scanned by the whole block, cell by cell; what is left is compared
+// by classes or sorted.  More
 // distinct cells than the hash holds: class by class of cells, from the
 // start (nothing but outputs, which come out the same, has been written).
 // (Out of line, so that its registers don't spill those of the common case;
@@ -791,7 +849,8 @@ __device__ __noinline__ void exec_long(const Src src, const u32 R, const BatchDe
     // ops a cell had before it was contended, two 16-bit counts a word (a
     // longer bucket than 65535 is not executed here)
     u32 *count = m.op();
-    __shared__ u32 s_distinct, s_con, s_left, s_cand[C::NW], s_row[C::RPT * C::NW], s_total;
+    u32 *cnt = m.cnt();
+    __shared__ u32 s_distinct, s_con, s_cand[C::NW], s_row[C::RPT * C::NW], s_total;
     __shared__ S s_sum[C::RPT * C::NW], s_all;
     const u32 tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -820,7 +879,8 @@ __device__ __noinline__ void exec_long(const Src src, const u32 R, const BatchDe
                 }
             src.template request<C>(lo + C::CHUNK, R, nx, nt);
             // ---- new cells, and their values before the batch ----
-            if (tid == 0) s_con = s_left = 0u;
+            if (tid == 0) s_con = 0u;
+            if (tid < C::NC) cnt[tid] = 0u;
 #pragma unroll
             for (int k = 0; k < C::RPT; k++) {
                 bool win = false, add1 = false;
@@ -889,20 +949,26 @@ __device__ __noinline__ void exec_long(const Src src, const u32 R, const BatchDe
                 const u32 c = __reduce_add_sync(FULL_MASK, (u32)__popc(con));
                 const u32 some = __ballot_sync(FULL_MASK, con != 0u);
                 cand = __shfl_sync(FULL_MASK, cand, some ? __ffs(some) - 1 : 0);
+                u32 here = 0;
+#pragma unroll
+                for (int k = 0; k < C::RPT; k++) here += (con >> k & 1u) && slot[k] == cand;
+                here = __reduce_add_sync(FULL_MASK, here);
                 if (lane == 0) {
                     if (c) atomicAdd(&s_con, c);
-                    s_cand[warp] = cand;
+                    s_cand[warp] = here >= kFew / C::NW ? cand : kEmpty;
                 }
             }
             __syncthreads();
             u32 left = s_con;
             // ---- frequent cells: an ordered scan each ----
+            int tries = 0;
 #pragma unroll 1
-            for (int h = 0; h < kHotTries && left > kFew; h++) {
-                const u32 sl = s_cand[h * (C::NW / kHotTries)];
+            for (int h = 0; h < C::NW && tries < kHotTries && left > kFew; h++) {
+                const u32 sl = s_cand[h];
                 bool seen = sl == kEmpty;
-                for (int j = 0; j < h; j++) seen = seen || s_cand[j * (C::NW / kHotTries)] == sl;
+                for (int j = 0; j < h; j++) seen = seen || s_cand[j] == sl;
                 if (seen) continue;  // the same for the block
+                tries++;
                 S sum[C::RPT];
                 u32 on = 0, rank[C::RPT];
 #pragma unroll
@@ -935,36 +1001,34 @@ __device__ __noinline__ void exec_long(const Src src, const u32 R, const BatchDe
                 left -= total;
                 __syncthreads();
             }
-            if (left > kFew) {
+            if (left) {
+                u32 rank[C::RPT];
 #pragma unroll
-                for (int k = 0; k < C::RPT; k++) {
-                    const u32 bal = __ballot_sync(FULL_MASK, con >> k & 1u);
-                    if (lane == 0) s_row[k * C::NW + warp] = (u32)__popc(bal);
-                }
-                scan_rows<C>(s_row, &s_total);
-#pragma unroll
-                for (int k = 0; k < C::RPT; k++) {
-                    const bool cn = con >> k & 1u;
-                    const u32 bal = __ballot_sync(FULL_MASK, cn);
-                    if (cn) cl[s_row[k * C::NW + warp] + __popc(bal & lanemask_lt())] = entry(slot[k], r[k].imm, op[k]);
-                }
-                run_sorted<C>(m, left, b, ctr, [&](u32 sl, V y) { val[sl] = y; });
-            } else if (left) {
-#pragma unroll
-                for (int k = 0; k < C::RPT; k++) {
-                    const bool cn = con >> k & 1u;
-                    const u32 bal = __ballot_sync(FULL_MASK, cn);
-                    if (!bal) continue;
-                    u32 at = 0;
-                    if (lane == 0) at = atomicAdd(&s_left, (u32)__popc(bal));
-                    at = __shfl_sync(FULL_MASK, at, 0) + (u32)__popc(bal & lanemask_lt());
-                    if (cn) cl[at] = entry(slot[k], r[k].imm, op[k]);
-                }
+                for (int k = 0; k < C::RPT; k++)
+                    if (con >> k & 1u) rank[k] = atomicAdd(&cnt[slot[k] / kClassSlots], 1u);
                 __syncthreads();
-                V y = 0;
-                const u32 sl = compare_all<C>(m, left, b, ctr, &y);
-                __syncthreads();
-                if (sl != kEmpty) val[sl] = y;
+                auto keep = [&](u32 sl, V y) { val[sl] = y; };
+                if (class_starts<C>(m)) {
+#pragma unroll
+                    for (int k = 0; k < C::RPT; k++)
+                        if (con >> k & 1u) cl[cnt[slot[k] / kClassSlots] + rank[k]] = entry(slot[k], r[k].imm, op[k]);
+                    __syncthreads();
+                    compare<C, true, false>(m, left, b, ctr, keep);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < C::RPT; k++) {
+                        const u32 bal = __ballot_sync(FULL_MASK, con >> k & 1u);
+                        if (lane == 0) s_row[k * C::NW + warp] = (u32)__popc(bal);
+                    }
+                    scan_rows<C>(s_row, &s_total);
+#pragma unroll
+                    for (int k = 0; k < C::RPT; k++) {
+                        const bool cn = con >> k & 1u;
+                        const u32 bal = __ballot_sync(FULL_MASK, cn);
+                        if (cn) cl[s_row[k * C::NW + warp] + __popc(bal & lanemask_lt())] = entry(slot[k], r[k].imm, op[k]);
+                    }
+                    run_sorted<C>(m, left, b, ctr, keep);
+                }
             }
             __syncthreads();
         }

@@ -68,6 +68,40 @@ def test_sizes_and_patterns(lib_loaded, n_ops, pattern):
         assert np.array_equal(ctx.download(t), ref)
 
 
+# Contended ops of a block around the edges between comparing them all, by
+# classes of slots, and sorting them; buckets that are executed first (more of
+# them than the list holds, some of them the first buckets anyway).
+@pytest.mark.parametrize("n_ops,n_hot,each", [
+    (1000, 1, 63), (1000, 2, 33), (2048, 8, 250), (2048, 1, 257), (2000, 1000, 2), (40000, 300, 40),
+    (40000, 100, 256), (40000, 60, 257), (150000, 40000, 3), (700001, 1, 3000), (700001, 31, 2500),
+    (700001, 33, 2000), (700001, 90, 2600)])
+def test_frequent_cells(lib_loaded, n_ops, n_hot, each):
+    rng = np.random.default_rng(n_ops + n_hot)
+    space = 1 << 20
+    # every other hot cell in a bucket of its own from the first on, the others anywhere
+    h = np.where(np.arange(n_hot) % 2 == 0, np.arange(n_hot) // 2 * (space // 608 + 1) % space, rng.integers(0, space, n_hot))
+    hot = (h * MIX_INVERSE) % space
+    cells = np.concatenate([np.repeat(hot, each), rng.integers(0, space, n_ops)])[:n_ops]
+    cells = cells[rng.permutation(n_ops)]
+    add = rng.random(n_ops) < 0.5
+    imm = np.where(add, rng.integers(-(1 << 19), 1 << 19, n_ops), 0)
+    opw = (add.astype(np.uint32) | ((imm & 0xFFFFF).astype(np.uint32) << np.uint32(12))).astype(np.uint32)
+    tf = np.unique(np.concatenate([[0, n_ops], rng.integers(0, n_ops + 1, n_ops // 5)])).astype(np.uint32)
+    with G.Context(device=0) as ctx:
+        t = ctx.create_table(space, 1)
+        ctx.fill_seeded(t, 9)
+        ref = O.table_init(9, space, 1)
+        b = ctx.batch(len(tf) - 1, n_ops)
+        for _ in range(2):
+            b.load(tf, cells.astype(np.uint64), opw)
+            b.execute()
+            commit, vals, st = b.results()
+            ref, rc, ro = O.replay(0, ref, tf, cells.astype(np.uint64), opw)
+            assert np.array_equal(commit, rc[:len(tf) - 1]) and np.array_equal(vals, ro)
+            assert (st.contended_ops, st.contended_cells, st.touched_words) == statistics(cells, add, 32)
+        assert np.array_equal(ctx.download(t), ref)
+
+
 @pytest.mark.parametrize("n_txns", [40, 300, 2500, 30000])
 @pytest.mark.parametrize("mode", [G.lib.MODE_STREAM, G.lib.MODE_GRAPH])
 def test_inserts_links_and_int64(lib_loaded, n_txns, mode):
