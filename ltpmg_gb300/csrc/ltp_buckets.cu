@@ -55,6 +55,7 @@ constexpr u32 inverse32(u32 a) {  // multiplicative inverse mod 2^32 (Newton)
 constexpr u32 kMixInv = inverse32(kMixMul);
 static_assert(kMixInv * kMixMul == 1u, "kMixMul is odd");
 
+constexpr u32 kSample = 8, kEarly = 32;  // see frequent_run
 constexpr u32 kOpBits = 11;  // an op's place in its tile
 
 // How a batch is split (host-made, passed by value).
@@ -74,6 +75,7 @@ struct BucketPlan {
     u32 word_shift;      // cells per conflict word (statistics only)
     u32 limit;           // a batch with a bucket longer than this is left to the conflict-word path (0: none)
     u32 hot;             // a tile's run of one bucket longer than this counts towards the limit
+    u32 often;           // a sampled tile's run longer than this speaks for a frequent cell
 };
 
 // Bijection on the cell numbers [0, 2^bits); equal parts of its range are the buckets.
@@ -187,6 +189,24 @@ __device__ __forceinline__ u32 block_excl(u32 v, u32 *s_w, u32 *total) {
 size_t part_smem(u32 tile, u32 buckets) {
     // records, then per-warp bucket counters (two to a word)
     return (size_t)tile * 8 + (size_t)(kPartBlock / 32) * ((buckets + 1) / 2) * 4;
+}
+
+// A tile's run of more than hot records of one bucket.  Only these are added
+// up: a bucket has at most tiles * hot <= limit / 2 records in its other runs,
+// so it is within the limit while its long runs stay within limit / 2.
+__device__ __forceinline__ void long_run(const BucketPlan &p, PartCounters *pc, u32 bucket, u32 len) {
+    if (atomicAdd(&pc->total[bucket], len) + len > p.limit / 2) pc->skew = 1u;
+}
+
+// Every kSample'th tile's runs that are long against the mean: buckets with
+// many of them are listed, to be executed first.  (All tiles' would be
+// kSample times the atomics: 2% of 1.8 M reads with many frequent cells.)
+__device__ __forceinline__ void frequent_run(PartCounters *pc, u32 bucket, u32 len) {
+    const u32 old = atomicAdd(&pc->sample[bucket], len);
+    if (old < kEarly && old + len >= kEarly) {
+        const u32 at = atomicAdd(&pc->n_first, 1u);
+        if (at < kMaxFirst) pc->first[at] = bucket;
+    }
 }
 
 // Two blocks per SM, not three: a tile's ops are held in registers from their
@@ -322,6 +342,7 @@ __global__ void __launch_bounds__(kPartBlock, 2) k_part(BatchDev b, TablesDev T,
     u32 all;
     u32 run = block_excl<NW>(tot, s_wsum, &all);
     uint16_t *row = p.offs + (u64)blockIdx.x * (B + 1);
+    const u32 often = blockIdx.x % kSample ? TILE : p.often;
     for (u32 q = q0; q < min(q0 + per, BW); q++) {
         u32 two = 0;
 #pragma unroll
@@ -336,13 +357,10 @@ __global__ void __launch_bounds__(kPartBlock, 2) k_part(BatchDev b, TablesDev T,
         }
         row[2 * q] = (uint16_t)run;
         if (2 * q + 1 < B) row[2 * q + 1] = (uint16_t)(run + c0);
-        // Only runs of more than hot records are added up: a bucket has at
-        // most tiles * hot = limit / 2 records in its other runs, so it is
-        // within the limit while its long runs stay within limit / 2.
-        if (p.limit) {
-            if (c0 > p.hot) atomicAdd(&pc->total[2 * q], c0), pc->hot = 1u;
-            if (c1 > p.hot) atomicAdd(&pc->total[2 * q + 1], c1), pc->hot = 1u;
-        }
+        if (c0 > p.hot) long_run(p, pc, 2 * q, c0);
+        if (c1 > p.hot) long_run(p, pc, 2 * q + 1, c1);
+        if (c0 > often) frequent_run(pc, 2 * q, c0);
+        if (c1 > often) frequent_run(pc, 2 * q + 1, c1);
         run += c0 + c1;
     }
     __syncthreads();
@@ -1195,6 +1213,26 @@ __device__ __forceinline__ void read_only(const BatchDev &b, const TablesDev &T,
     }
 }
 
+// The bucket of a block when some are listed to be executed first: the first
+// blocks take the listed ones, whose own blocks take the buckets that the
+// first ones left, in order.  (Full warps.)
+__device__ __forceinline__ u32 first_order(const PartCounters *pc, u32 block) {
+    const u32 lane = threadIdx.x & 31, m = min(pc->n_first, kMaxFirst);
+    const u32 h = lane < m ? pc->first[lane] : 0xFFFFFFFFu;
+    // of the first m buckets those that are not listed; of the listed ones those beyond
+    u32 left = ~__reduce_or_sync(FULL_MASK, h < 32u ? 1u << h : 0u) & (m == 32u ? FULL_MASK : (1u << m) - 1u);
+    const u32 beyond = __ballot_sync(FULL_MASK, lane < m && h >= m), me = __ballot_sync(FULL_MASK, h == block);
+    if (block < m) return __shfl_sync(FULL_MASK, h, (int)block);
+    if (!me) return block;
+    for (u32 k = (u32)__popc(beyond & (me - 1u)); k; k--) left &= left - 1u;
+    return (u32)__ffs((int)left) - 1u;
+}
+
+// One block per bucket, two per SM: a block is a chain of latencies (offsets,
+// records, cells, outputs) under which the other one executes.  A bucket with
+// a frequent cell is several chunks long: started with the last wave, order
+// entry's sixteen (5,000 records each) kept the kernel at 157 us for 1.4 M
+// ops, started first 110 (the case 437 -> 372 us).
 template <class C>
 __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T, BucketPlan p) {
     pdl_begin();
@@ -1209,46 +1247,48 @@ __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T,
     const bool extra = blockIdx.x == p.n_buckets;  // with inserts: one block more
     TileSrc src;
     src.recs = p.recs;
-    const uint16_t *offs = p.offs + blockIdx.x;  // the bucket's column
     src.ops = Smem<C>().op();
     src.pre = Smem<C>().pre();
     src.adj = Smem<C>().adj();
     src.n_tiles = p.n_tiles;
     src.tile = p.tile;
     const u32 per = (p.n_tiles + C::BLOCK - 1) / C::BLOCK;
-    u32 at[TPT], cnt[TPT], len = 0, R;
+    u32 at[TPT], cnt[TPT], len = 0, R, bucket = blockIdx.x;
     u64 x[TPT][PRE];
+    auto column = [&]() {
+        len = 0;
 #pragma unroll
-    for (int j = 0; j < TPT; j++) {
-        const u32 t = tid * per + (u32)j;
-        at[j] = cnt[j] = 0;
-        if (!extra && (u32)j < per && t < p.n_tiles) {
-            const uint16_t *o = offs + (u64)t * (p.n_buckets + 1);
-            at[j] = o[0];
-            cnt[j] = o[1] - at[j];
+        for (int j = 0; j < TPT; j++) {
+            const u32 t = tid * per + (u32)j;
+            at[j] = cnt[j] = 0;
+            if (!extra && (u32)j < per && t < p.n_tiles) {
+                const uint16_t *o = p.offs + (u64)t * (p.n_buckets + 1) + bucket;
+                at[j] = o[0];
+                cnt[j] = o[1] - at[j];
+            }
+            len += cnt[j];
         }
-        len += cnt[j];
-    }
+    };
+    column();
     // (kernel-uniform: nobody writes these now; both counters' flags, so that
     // the loads don't wait for one another)
     const u32 stamp = p.state->stamp2, par = p.state->par2;
-    const u32 w0 = p.ctr[0].writes, w1 = p.ctr[1].writes, h0 = p.ctr[0].hot, h1 = p.ctr[1].hot;
+    const u32 w0 = p.ctr[0].writes, w1 = p.ctr[1].writes, k0 = p.ctr[0].skew, k1 = p.ctr[1].skew;
+    const u32 f0 = p.ctr[0].n_first, f1 = p.ctr[1].n_first;
     const int e0 = p.ctr[0].c.err, e1 = p.ctr[1].c.err;
     PartCounters *pc = p.ctr + par;
-    const u32 writes = par ? w1 : w0, hot = par ? h1 : h0;
+    const u32 writes = par ? w1 : w0, skew = writes && (par ? k1 : k0);
     const int err = par ? e1 : e0;
+    if (par ? f1 : f0) {
+        bucket = first_order(pc, bucket);
+        if (bucket != blockIdx.x) column();
+    }
 #pragma unroll
     for (int j = 0; j < TPT; j++)
 #pragma unroll
         for (int i = 0; i < PRE; i++)
             if (writes && (u32)i < cnt[j]) x[j][i] = __ldcs(&p.recs[(u64)(tid * per + (u32)j) * p.tile + at[j] + (u32)i]);
     const bool room = !b.payload_len || !no_room(T, pc->c.ins_total);
-    u32 skew = 0;
-    if (hot && p.limit) {  // is some bucket too long for one block?
-        bool over = false;
-        for (u32 i = tid; i < p.n_buckets; i += C::BLOCK) over |= pc->total[i] > p.limit / 2;
-        skew = __syncthreads_or(over);
-    }
     if (blockIdx.x == 0 && tid == 0) {
         p.state->stamp1 = stamp;
         p.state->par1 = par ^ 1u;
@@ -1273,7 +1313,7 @@ __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T,
     } else {
         u32 pos = block_excl<C::NW>(len, s_w, &R);
         src.cell_bits = p.cell_bits;
-        src.start = blockIdx.x * p.width;
+        src.start = bucket * p.width;
         if (R > C::CHUNK) {
             u32 *pre = Smem<C>().pre(), *adj = Smem<C>().adj();
 #pragma unroll
@@ -1506,7 +1546,10 @@ bool plan_buckets(const Launch &L, const BatchDev &b, const TablesDev &T, const 
     p->tile = tile;
     p->n_tiles = (n + tile - 1) / tile;
     p->limit = n > kBucketLimit ? kBucketLimit : 0;
-    p->hot = kBucketLimit / 2 / p->n_tiles;
+    p->hot = p->limit ? kBucketLimit / 2 / p->n_tiles : tile;
+    // Runs of more than twice the mean and five ops are rare by chance; within
+    // one wave every bucket starts at once and none need be known.
+    p->often = nb > wave ? 2 * tile / nb + 5 : tile;
     // the fallback counts touched words of 32 cells
     if (p->limit && p->word_shift != 5) return false;
     return p->n_tiles <= kMaxTiles && (u64)p->n_tiles * (nb + 1) * 2 <= s.cap_ops * 8 && (u64)p->n_tiles * tile <= s.cap_ops;

@@ -120,11 +120,15 @@ struct PartState {
     u32 bar[2];        // grid barrier of the fallback launch
 };
 constexpr u32 kMaxBuckets = 1536;  // four waves and more of two blocks per SM
+constexpr u32 kMaxFirst = 32;
 struct PartCounters {
     Counters c;              // err, bad_op and the insert counts
     u32 writes;              // some op writes an existing cell
-    u32 hot;                 // some bucket has long runs ...
-    u32 total[kMaxBuckets];  // ... this many records of them per bucket
+    u32 skew;                // some bucket is too long for one block
+    u32 n_first;             // buckets to be executed first (may count on) ...
+    u32 first[kMaxFirst];    // ... and which
+    u32 total[kMaxBuckets];  // records of each bucket in long runs,
+    u32 sample[kMaxBuckets]; // and in runs longer than usual of some tiles
 };
 
 // Scratch owned by the context, sized by the cell space and the batch capacity.
