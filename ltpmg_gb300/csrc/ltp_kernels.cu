@@ -1480,9 +1480,14 @@ __global__ void __launch_bounds__(kInsPrefixBlock) k_ins_prefix(BatchDev b, Tabl
 // by the row reads.  Reading every cell straight from its row, a sector per 4
 // bytes, the insert kernel took 76 us for 1.38 M order-entry ops, 26 us for
 // 1.8 M YCSB-E ops and 39 us for the 31,500 ops of a small order-entry call;
-// this one 47, 22 and 17 us (512 threads x 4 ops, two blocks per SM; 256 x 8
-// with three: 3% slower on order entry, 3% faster on YCSB-E).
-constexpr u32 kRowsBlock = 512, kRowsIpt = 4, kRowsTile = kRowsBlock * kRowsIpt;
+// this one 47, 22 and 17 us (512 threads x 4 ops, two blocks per SM).
+//
+// Where rows are few (YCSB-E: one row of three columns per 55 ops) a slice is the
+// chain alone, and three blocks of 256 threads x 8 ops take it better: 3.6 M
+// YCSB-E ops 44 -> 40 us, the read-only case with inserts 161 -> 156; order
+// entry, whose rows keep the block busy, 372 -> 385.  The line, a payload slot
+// per four ops, lies between the two (0.05 and 4 slots per op).
+constexpr u32 kRowsTile = 2048;
 constexpr u32 kRowsStage = 11264;  // 4-byte slots staged at a time
 constexpr u32 kRowsSmem = kRowsStage * 4 + kRowsTile * 4;
 static_assert(kInsTile == 2 * kRowsTile, "an insert tile is two of these");
@@ -1494,8 +1499,10 @@ __device__ __forceinline__ void copy_async4(u32 *dst, const int32_t *src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__global__ void __launch_bounds__(kRowsBlock, 2) k_rows(BatchDev b, TablesDev T, Scratch s, Counters *ctr,
-                                                        const PartState *ps) {
+template <int kRowsBlock, int MINB>
+__global__ void __launch_bounds__(kRowsBlock, MINB) k_rows(BatchDev b, TablesDev T, Scratch s, Counters *ctr,
+                                                           const PartState *ps) {
+    constexpr u32 kRowsIpt = kRowsTile / kRowsBlock;
     pdl_begin();
     if (ps) {  // bucket path: its current counters; nothing to do for a batch it left or refused
         if (ps->skew || ps->full) return;
@@ -1893,18 +1900,26 @@ static void pick_front(const Tuning &t, front_fn *mark, front_fn *classify) {
 
 static int capped(int grid, u64 upper) { return (int)((u64)grid < upper ? (u64)grid : (upper ? upper : 1)); }
 
+template <int BLOCK, int MINB>
+static cudaError_t go_rows(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
+                           const PartState *ps) {
+    static int grid = 0, sms = 0;
+    if (sms != L.num_sms) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_rows<BLOCK, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
+        if (e != cudaSuccess) return e;
+        grid = occ_grid(k_rows<BLOCK, MINB>, BLOCK, L.num_sms, kRowsSmem);
+        sms = L.num_sms;
+    }
+    return launch_k(L.pdl, k_rows<BLOCK, MINB>, capped(grid, (b.n_ops + kRowsTile - 1) / kRowsTile), BLOCK, kRowsSmem, L.stream,
+                    b, T, s, ctr, ps);
+}
+
 cudaError_t launch_insert(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
                           int prefixed, const PartState *ps) {
     if (prefixed) {
-        static int grows = 0, rsms = 0;
-        if (rsms != L.num_sms) {
-            const cudaError_t e = cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
-            if (e != cudaSuccess) return e;
-            grows = occ_grid(k_rows, (int)kRowsBlock, L.num_sms, kRowsSmem);
-            rsms = L.num_sms;
-        }
-        return launch_k(L.pdl, k_rows, capped(grows, (b.n_ops + kRowsTile - 1) / kRowsTile), kRowsBlock, kRowsSmem, L.stream, b,
-                        T, s, ctr, ps);
+        // few rows per op: see k_rows
+        return b.payload_len < b.n_ops / 4 ? go_rows<256, 3>(L, b, T, s, ctr, ps) : go_rows<512, 2>(L, b, T, s, ctr, ps);
     }
     static int gins = 0, sms = 0;
     if (sms != L.num_sms) {

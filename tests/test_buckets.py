@@ -204,3 +204,41 @@ def test_rows_of_every_width(lib_loaded, n_txns):
     assert np.array_equal(vals, ro)
     for k in range(len(shapes)):
         assert np.array_equal(finals[k], after[k][0][:, :after[k][1]]), k
+
+
+@pytest.mark.parametrize("n_txns,reads", [(1, 700), (12, 700), (700, 700), (4000, 600), (300, 4)])
+def test_few_rows_per_op(lib_loaded, n_txns, reads):
+    """Inserts, linked and not, among many reads (both shapes of the insert
+    kernel; insert tiles with no insert, one and a few)."""
+    rng = np.random.default_rng(n_txns)
+    shapes = [(64, (1 << 64) - 1), (3, 0), (17, 1 << 16)]
+    slots = np.array([c + bin(m).count("1") for c, m in shapes])
+    t = rng.integers(0, len(shapes), n_txns)
+    link = rng.random(n_txns) < 0.5
+    first = np.concatenate([[0], np.cumsum(slots[t])])
+    kinds = rng.integers(0, 50, (n_txns, reads + 1)).astype(np.uint64)
+    keys = np.concatenate([kinds, first[:-1, None].astype(np.uint64)], axis=1).reshape(-1)
+    opw = np.full((n_txns, reads + 2), G.opword(G.OP_READ, 5, 0), np.uint32)
+    opw[:, reads] = [G.opword(G.OP_ADD, 7, 0, int(v)) for v in rng.integers(-99, 99, n_txns)]
+    opw[:, reads + 1] = [G.opword(G.OP_INSERT, 2, int(x), int(li)) for x, li in zip(t, link)]
+    opw = opw.reshape(-1)
+    pay = rng.integers(-(1 << 31), 1 << 31, int(first[-1])).astype(np.int32)
+    assert (len(pay) < len(opw) // 4) == (reads > 100)
+    tf = np.arange(0, len(opw) + 1, reads + 2, dtype=np.uint32)
+    rows = [50 + int((t == k).sum()) for k in range(len(shapes))]
+    with G.Context(device=0) as ctx:
+        for k, (c, m) in enumerate(shapes):
+            ctx.create_table(50, c, rows_cap=rows[k], wide=[j for j in range(c) if m >> j & 1])
+            ctx.fill_seeded(k, 11)
+        tabs = [(np.concatenate([ctx.download(k), np.zeros((c, rows[k] - 50), np.int64 if m else np.int32)], axis=1), 50, m)
+                for k, (c, m) in enumerate(shapes)]
+        b = ctx.batch(n_txns, len(keys))
+        b.load(tf, keys, opw)
+        b.load_payload(pay)
+        b.execute()
+        _, vals, _ = b.results64()
+        finals = [ctx.download(k) for k in range(len(shapes))]
+    after, _, ro = O.replay_tables(0, tabs, tf, keys, opw, pay)
+    assert np.array_equal(vals, ro)
+    for k in range(len(shapes)):
+        assert np.array_equal(finals[k], after[k][0][:, :after[k][1]]), k
