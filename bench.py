@@ -62,11 +62,47 @@ KERNEL_BYTES = {  # st["key_bytes"]: 8, or 4 for batches loaded with 32-bit keys
     "insert": lambda st: st.get("insert_bytes", 0),
     "finish": lambda st: 12 * st["touched_words"],
 }
+# Ordered-rule batches of up to 2^21 ops execute by buckets of cells
+# (ltp_buckets.cu): the split kernel is timed as stage "mark", the bucket
+# kernel as "apply"; per op a record written and read, the cell read, the
+# output written (written cells come on top and are not counted).
+BUCKET_OPS = 2 << 20
+BUCKET_BYTES = {
+    "split": ("mark", lambda st: (12 + st["key_bytes"]) * st["ops"]),
+    "bucket": ("apply", lambda st: 16 * st["ops"]),
+    "insert": ("insert", lambda st: st.get("insert_bytes", 0)),
+}
+
+
+def mean_counters(stats):
+    return {k: sum(s[k] for s in stats) / len(stats) for k in ("ops", "touched_words", "contended_cells", "contended_ops")}
+
+
+def stage_report(stats, extra):
+    """Average kernel times, algorithmic bytes per launch and mean counters
+    of the batches of the path (conflict words or buckets) that takes more
+    of the time; extra: further counters."""
+    groups = {True: [], False: []}
+    for s in stats:
+        groups[s["ops"] <= BUCKET_OPS].append(s)
+    by_buckets = max(groups, key=lambda k: sum(sum(s["ms_stage"].values()) for s in groups[k]))
+    g = groups[by_buckets]
+    mean = dict(mean_counters(g), **extra)
+    kernels = BUCKET_BYTES if by_buckets else {k: (k, f) for k, f in KERNEL_BYTES.items()}
+    avg = {k: sum(s["ms_stage"][stage] for s in g) / len(g) for k, (stage, _) in kernels.items()}
+    return by_buckets, avg, {k: f(mean) for k, (_, f) in kernels.items()}, mean
+
+
 def kernels_per_batch(n_ops, has_payload):
-    """Kernels one batch launches under the ordered rule: mark, ids, dbase,
+    """Kernels one batch launches under the ordered rule.  By buckets: split
+    (not for one block's batch) and bucket, the insert kernel and the closing
+    one with a payload, and from 32,768 ops on the fallback for skewed
+    batches.  By conflict words: mark, ids, dbase,
     classify, one radix pass per 8 bits of the largest possible contended id
     (n_ops - 1), apply, the insert prefix and insert (only with a payload),
     finish."""
+    if n_ops <= BUCKET_OPS:
+        return (1 if n_ops <= 2048 else 2) + (2 if has_payload else 0) + (1 if n_ops > 32767 else 0)
     passes = 1
     while passes < 4 and ((max(n_ops, 1) - 1) >> (8 * passes)) != 0:
         passes += 1
@@ -498,18 +534,17 @@ def run_ours(args, config):
             "kernel_timing_pass_ms_per_step": ms_timed / max(1, min(args.steps, 5)),
             "pipeline": {"algorithmic_bytes_per_step": alg, "avg_step_ms": step_ms,
                          "achieved": alg / (step_ms / 1e3) / 1e9, "frac": alg / (step_ms / 1e3) / 1e9 / peak}}
-    mean_stats = {k: sum(s[k] for s in stats) / len(stats) for k in ("ops", "touched_words", "contended_cells",
-                                                                     "contended_ops")}
-    mean_stats["key_bytes"] = key_bytes
+    mean_stats = mean_counters(stats)
     if mode != G.MODE_PERSISTENT:
-        avg = {name: sum(s["ms_stage"][name] for s in stats) / len(stats) for name in KERNEL_BYTES}
+        by_buckets, avg, kernel_bytes, path_stats = stage_report(stats, {"key_bytes": key_bytes})
         dom = max(avg, key=avg.get)
-        dom_bytes = KERNEL_BYTES[dom](mean_stats)
+        dom_bytes = kernel_bytes[dom]
         achieved = dom_bytes / (avg[dom] / 1e3) / 1e9
-        traffic_b = measured_traffic(config, dom, mean_stats)
+        traffic_b = measured_traffic(config, dom, path_stats)
         roof.update({"kernel": dom, "achieved": achieved, "frac": achieved / peak, "traffic": traffic_b,
-                     "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": avg[dom], "kernel_ms": avg,
-                     "random_access": random_access_roof(G, local, sh, mean_stats, avg, config)})
+                     "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": avg[dom], "kernel_ms": avg})
+        if not by_buckets:
+            roof["random_access"] = random_access_roof(G, local, sh, path_stats, avg, config)
     else:
         roof.update({"kernel": "k_persist (whole pipeline, one launch per step)", "achieved":
                      roof["pipeline"]["achieved"], "frac": roof["pipeline"]["frac"], "traffic": None,
@@ -828,17 +863,15 @@ def run_payload(args, config):
             "kernel_timing_pass_ms_per_step": ms_timed / timing_steps,
             "pipeline": {"algorithmic_bytes_per_step": alg, "avg_step_ms": step_ms,
                          "achieved": alg / (step_ms / 1e3) / 1e9, "frac": alg / (step_ms / 1e3) / 1e9 / peak}}
-    mean_stats = {k: sum(s[k] for s in stats) / len(stats) for k in ("ops", "touched_words", "contended_cells",
-                                                                     "contended_ops")}
-    mean_stats["insert_bytes"] = sum(wl.insert_bytes(h) for h in host) / len(host)
-    mean_stats["key_bytes"] = 4
+    mean_stats = mean_counters(stats)
     if mode != G.MODE_PERSISTENT:
-        avg = {nm: sum(s["ms_stage"][nm] for s in stats) / len(stats) for nm in KERNEL_BYTES}
+        _, avg, kernel_bytes, path_stats = stage_report(
+            stats, {"insert_bytes": sum(wl.insert_bytes(h) for h in host) / len(host), "key_bytes": 4})
         dom = max(avg, key=avg.get)
-        dom_bytes = KERNEL_BYTES[dom](mean_stats)
+        dom_bytes = kernel_bytes[dom]
         achieved = dom_bytes / (avg[dom] / 1e3) / 1e9
         roof.update({"kernel": dom, "achieved": achieved, "frac": achieved / peak,
-                     "traffic": measured_traffic(config, dom, mean_stats),
+                     "traffic": measured_traffic(config, dom, path_stats),
                      "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": avg[dom], "kernel_ms": avg})
     else:
         roof.update({"kernel": "k_persist (whole pipeline, one launch per step)",

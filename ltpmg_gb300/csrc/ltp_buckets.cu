@@ -5,31 +5,33 @@
 // every bucket is executed by one block in shared memory:
 //
 //   part    each block takes one tile of the batch: decodes and checks its
-//           ops, ranks them by bucket in op order (match.any per warp,
-//           per-warp counters) and writes the tile's records grouped by
-//           bucket into the tile's own place, with the tile's bucket offsets
-//           -- no global histogram, no look-back, no atomics per op
+//           ops, ranks them by bucket in op order (per-warp counters in shared
+//           memory) and writes the tile's records grouped by bucket into the
+//           tile's own place, with the tile's bucket offsets -- no global
+//           histogram, no look-back, no atomics per op
 //   bucket  one block per bucket reads the bucket's run from every tile (so
 //           its records arrive in op order), finds the distinct cells in a
 //           shared-memory hash, reads each cell once, executes what is not
-//           contended, sorts what is by its hash slot (two 6- or 7-bit passes
-//           in shared memory), scans the increments and writes each written
-//           cell once.  A bucket longer than a chunk is executed chunk by
-//           chunk, the cells' values carried in shared memory; a bucket with
-//           more distinct cells than the hash holds is split into classes.
+//           contended, resolves what is (compared by classes of hash slots,
+//           or sorted and scanned) and writes each written cell once.  A
+//           bucket longer than a chunk is executed chunk by chunk, the cells'
+//           values carried in shared memory; a bucket with more distinct cells
+//           than the hash holds is split into classes of cells.
 //   solo    a batch of at most kSoloOps ops: the bucket kernel on the whole
 //           batch, straight from its arrays, as one launch
 //
 // Against the conflict-word path (ltp_kernels.cu) there is no state per cell
 // of the table to mark, scan and clear, each op's key and opword are read
-// once, and a batch takes two launches instead of eleven.  Measured on one
-// GB300, per batch: 640 ops (a synchronous call, copies included) 77 -> 47
-// us; 65,536 ops in a graph 64 -> 20 us; 655,360 uniform ops over 2^20 x 10
-// cells 92 -> 44 us; 32,768 x 55 read-only ops with inserts 99 -> 87 us.
-// What bounds it: random sectors between the SMs and L2 -- per op one read of
-// its cell, one atomic for the touched-word count and one store of its value
-// (655,360 ops: 2.8 + 4.9 + 3.3 us at the measured rates) -- and, with two
-// blocks of 512 threads per SM, the chain of their latencies.
+// once, and a batch takes two launches (with the skew fallback's gate three)
+// instead of eleven.  Measured on one GB300, per batch: 640 ops (a synchronous
+// call, copies included) 77 -> 27 us; 17,000 to 270,000 ops in a list 64 -> 17
+// us; 655,360 uniform ops over 2^20 x 10 cells 92 -> 42 us; 1.4 M order-entry
+// ops with inserts 269 -> 186 us; 32,768 x 55 read-only ops with inserts 99 ->
+// 80 us.  What bounds it: random sectors between the SMs and L2 -- per op one
+// read of its cell, one atomic for the touched-word count and one store of its
+// value (655,360 ops: 2.8 + 4.9 + 3.3 us at the measured rates, of 13 us in
+// part and 34 in bucket) -- and, with two blocks of 512 threads per SM, the
+// chain of their latencies.
 #include <stdint.h>
 #include <string.h>
 
@@ -1218,6 +1220,7 @@ __device__ __forceinline__ void read_only(const BatchDev &b, const TablesDev &T,
 // blocks take the listed ones, whose own blocks take the buckets that the
 // first ones left, in order.  (Full warps.)
 __device__ __forceinline__ u32 first_order(const PartCounters *pc, u32 block) {
+    static_assert(kMaxFirst == 32, "a lane per listed bucket");
     const u32 lane = threadIdx.x & 31, m = min(pc->n_first, kMaxFirst);
     const u32 h = lane < m ? pc->first[lane] : 0xFFFFFFFFu;
     // of the first m buckets those that are not listed; of the listed ones those beyond

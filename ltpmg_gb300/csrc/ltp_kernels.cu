@@ -20,6 +20,10 @@
 //   finish    clears exactly the bitmap words and look-back slots the batch
 //             used, so the next batch starts clean
 //
+// Ordered-rule batches of at most 2^21 ops execute by buckets of cells
+// instead (ltp_buckets.cu); these kernels take the larger ones, the priority
+// rule, the persistent mode, skewed batches and every batch's inserts.
+//
 // This replaces the reference's nine-stage pipeline (register, prefix,
 // bitmap compaction, per-row scatter, per-row merge sort, per-row serial
 // commit: cuda/src/gpulauncher.cu:755-1116) while keeping its rule that all
