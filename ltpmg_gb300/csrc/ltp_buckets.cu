@@ -27,7 +27,7 @@
 // call, copies included) 77 -> 27 us; 17,000 to 270,000 ops in a list 64 -> 17
 // us; 655,360 uniform ops over 2^20 x 10 cells 92 -> 42 us; 1.4 M order-entry
 // ops with inserts 269 -> 186 us; 32,768 x 55 read-only ops with inserts 99 ->
-// 80 us.  What bounds it: random sectors between the SMs and L2 -- per op one
+// 78 us.  What bounds it: random sectors between the SMs and L2 -- per op one
 // read of its cell, one atomic for the touched-word count and one store of its
 // value (655,360 ops: 2.8 + 4.9 + 3.3 us at the measured rates, of 13 us in
 // part and 34 in bucket) -- and, with two blocks of 512 threads per SM, the
@@ -680,7 +680,7 @@ __device__ __forceinline__ bool class_starts(const Smem<C> &m) {
 //
 // Bound by instruction issue: all of a chunk's ops against all took a third of
 // a block's time on order entry (250 ops: 13,000 cycles), by classes of eight
-// slots an op meets a handful of others (order entry 461 -> 437 us, six
+// slots an op meets a handful of others (order entry 461 -> 444 us, six
 // batches of 327,680 ops in the pipeline 307 -> 276, 1.5 M uniform ops 92 ->
 // 74; classes of sixteen the same).  The classes' scan costs two barriers: up
 // to kTiny ops do without (3,000 ops 9.7 -> 9.2 us, uneven batches 207 -> 201
@@ -1236,7 +1236,7 @@ __device__ __forceinline__ u32 first_order(const PartCounters *pc, u32 block) {
 // records, cells, outputs) under which the other one executes.  A bucket with
 // a frequent cell is several chunks long: started with the last wave, order
 // entry's sixteen (5,000 records each) kept the kernel at 157 us for 1.4 M
-// ops, started first 110 (the case 437 -> 372 us).
+// ops, started first 99 (the case 444 -> 372 us).
 template <class C>
 __global__ void __launch_bounds__(C::BLOCK, 2) k_bucket(BatchDev b, TablesDev T, BucketPlan p) {
     pdl_begin();
