@@ -108,8 +108,8 @@ int ensure_scratch(ltp_ctx *ctx, uint64_t n_ops) {
         CK(dalloc(&s.cview, words + 1));  // 8 B per 32 cells; the 64-cell view takes 16 B per word
         CK(cudaMemset(s.cview, 0, (words + 1) * sizeof(uint2)));
         CK(dalloc(&s.word_epoch, words));
-        CK(cudaMemset(s.word_epoch, 0, words * 4));
-        CK(cudaMemset(s.pstate, 0, sizeof(PartState)));  // the stamps start over
+        s.n_words = words;
+        CK(launch_reset_buckets(cudaStreamLegacy, s));  // the stamps start over
         CK(cudaStreamSynchronize(cudaStreamLegacy));
         ctx->scratch_gen++;
         ctx->alloc_words = words;

@@ -2229,12 +2229,17 @@ cudaError_t launch_reset_scratch(cudaStream_t st, const Scratch &s) {
     cudaMemsetAsync(s.st_apply, 0, s.cap_tiles * 8, st);
     cudaMemsetAsync(s.st_ins, 0, s.cap_tiles * LTP_MAX_TABLES * 4, st);
     if (s.ins_pre != s.st_ins) cudaMemsetAsync(s.ins_pre, 0, s.cap_tiles * LTP_MAX_TABLES * 4, st);
-    if (s.pctr) {
-        cudaMemsetAsync(s.pctr, 0, 2 * sizeof(PartCounters), st);
-        cudaMemsetAsync(s.fctr, 0, sizeof(Counters), st);
-        cudaMemsetAsync(s.pstate, 0, sizeof(PartState), st);
-        cudaMemsetAsync(s.word_epoch, 0, s.n_words * 4, st);
-    }
+    if (s.pctr) return launch_reset_buckets(st, s);
+    return cudaGetLastError();
+}
+
+// All of it together: the state says which counters the next batch finds
+// clean, and its stamps are compared with the words'.
+cudaError_t launch_reset_buckets(cudaStream_t st, const Scratch &s) {
+    cudaMemsetAsync(s.pctr, 0, 2 * sizeof(PartCounters), st);
+    cudaMemsetAsync(s.fctr, 0, sizeof(Counters), st);
+    cudaMemsetAsync(s.pstate, 0, sizeof(PartState), st);
+    cudaMemsetAsync(s.word_epoch, 0, s.n_words * 4, st);
     return cudaGetLastError();
 }
 
