@@ -138,7 +138,7 @@ __device__ __forceinline__ bool op_cell(const TablesDev &T, const u64 *s_rows, u
 // An insert op's checks (it has no cell).
 __device__ __forceinline__ bool insert_valid(const BatchDev &b, const TablesDev &T, u64 key, u64 i, u32 w) {
     const u32 tb = opw_table(w);
-    return tb < T.n && key + insert_slots(T.t[tb]) <= b.payload_len && insert_link_ok(b, T.t[tb], i, w);
+    return tb < T.n && payload_row_fits(key, insert_slots(T.t[tb]), b.payload_len) && insert_link_ok(b, T.t[tb], i, w);
 }
 
 __device__ __forceinline__ void set_bad(Counters *ctr, u64 i) {
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kPartBlock, 2) k_part(BatchDev b, TablesDev T,
             if (ins >> k & 1u) {
                 const u64 i = wbase + (u64)k * 32 + lane;
                 const u32 tb = opw_table(w[k]), d = insert_link(w[k]);
-                bool ok = tb < T.n && key[k] + insert_slots(T.t[tb]) <= b.payload_len;
+                bool ok = tb < T.n && payload_row_fits(key[k], insert_slots(T.t[tb]), b.payload_len);
                 if (ok && d) ok = opw_col(w[k]) < T.t[tb].n_cols && d <= i && i - d >= first[k] && opw_kind(linked[k]) <= LTP_OP_ADD;
                 if (ok) atomicAdd(&s_ins[tb], 1u);
                 else set_bad(&pc->c, i);

@@ -4,6 +4,7 @@
 #pragma once
 #include <stdint.h>
 
+#include "ltp_bounds.h"
 #include "ltp_internal.cuh"
 
 namespace ltp {

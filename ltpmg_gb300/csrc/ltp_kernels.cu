@@ -263,7 +263,8 @@ __device__ __forceinline__ void phase_mark(const BatchDev &b, const TablesDev &T
             if (i >= n) continue;
             if (opw_kind(w[k]) == LTP_OP_INSERT) {  // appends a row: no existing cell to mark
                 const u32 tb = opw_table(w[k]);
-                if (tb < T.n && key[k] + insert_slots(T.t[tb]) <= b.payload_len && insert_link_ok(b, T.t[tb], i, w[k])) {
+                if (tb < T.n && payload_row_fits(key[k], insert_slots(T.t[tb]), b.payload_len) &&
+                    insert_link_ok(b, T.t[tb], i, w[k])) {
                     atomicAdd(&s_ins[tb], 1u);
                 } else {
                     atomicMax(&ctr->bad_op, ~i);

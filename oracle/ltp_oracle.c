@@ -398,7 +398,7 @@ static int check_op_t(uint32_t n_tables, const ltpo_table *T, uint64_t i, uint64
     if (kind == 2) {
         const uint64_t slots = T[tb].n_cols + popc64(T[tb].wide);
         const uint32_t d = (uint32_t)LTPO_IMM(w) & 0x3FFu;
-        if (keys[i] + slots > payload_len) return -1;
+        if (slots > payload_len || keys[i] > payload_len - slots) return -1; /* (key + slots may wrap) */
         if (d && (LTPO_COL(w) >= T[tb].n_cols || d > i - first || LTPO_KIND(opw[i - d]) > 1)) return -1;
         return 0;
     }
