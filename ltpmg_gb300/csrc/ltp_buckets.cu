@@ -249,6 +249,9 @@ __global__ void __launch_bounds__(kPartBlock, 2) k_part(BatchDev b, TablesDev T,
         if (tid == 0) {
             p.state->stamp2 = stamp + 1u;
             p.state->par2 = par;
+            p.state->skew = 0u;  // (set still after a fallback that gave up)
+            p.state->joined = p.state->members = p.state->left = 0u;
+            p.state->bar[0] = 0u;
         }
     }
     commit_all(b, blockIdx.x, gridDim.x);

@@ -57,6 +57,13 @@ __device__ __forceinline__ u32 ld_status32(const u32 *p) {
 __device__ __forceinline__ void st_status32(u32 *p, u32 v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// The blocks among which a phase's work is spread: a launch's own, or those of
+// them that take part.
+struct Grid {
+    u32 id, n;  // this block's number, their number
+};
+__device__ __forceinline__ Grid whole_grid() { return Grid{blockIdx.x, gridDim.x}; }
+
 __device__ __forceinline__ u32 lanemask_lt() {
     u32 m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));

@@ -117,7 +117,10 @@ struct PartState {
     u32 stamp2, par2;  // stamp: batches executed, marks the conflict words a batch touched
     u32 skew;          // the batch at hand has an overlong bucket: left to the conflict-word path
     u32 full;          // the batch at hand found no room for its inserts
-    u32 bar[2];        // grid barrier of the fallback launch
+    // the fallback launch, zero before it: blocks that joined it (top bit: no
+    // more may), how many take part, how many of them are done, their barrier
+    u32 joined, members, left;
+    u32 bar[2];
 };
 constexpr u32 kMaxBuckets = 1536;  // four waves and more of two blocks per SM
 constexpr u32 kMaxFirst = 32;
@@ -201,7 +204,7 @@ cudaError_t launch_execute(const Launch &L, const BatchDev &b, const TablesDev &
 bool launch_buckets(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *snap,
                     cudaError_t *status);
 // Pieces of the conflict-word path that the bucket path uses: the insert
-// kernel, and the persistent kernel on one batch, run only when
+// kernel, and the persistent kernel's phases on one batch, run only when
 // s.pstate->skew is set.
 cudaError_t launch_insert(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
                           int prefixed, const PartState *ps);

@@ -205,7 +205,8 @@ constexpr size_t mark_smem_bytes() { return 2ull * BLOCK * IPT * (4 + 3 * (WB / 
 constexpr u64 kStreamOpsBytes = 96ull << 20;
 
 template <int BLOCK, int IPT, int WB>
-__device__ __forceinline__ void phase_mark(const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr) {
+__device__ __forceinline__ void phase_mark(const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
+                                           const Grid g) {
     typedef typename Wd<WB>::T WT;
     // A batch with at least twice as many ops as conflict words touches
     // most of them: ids and finish will visit every word in address order,
@@ -239,7 +240,7 @@ __device__ __forceinline__ void phase_mark(const BatchDev &b, const TablesDev &T
         s_whi1[warp] = 0u;
     }
     if (threadIdx.x == 0) s_wide = 0u;
-    for (u64 base = (u64)blockIdx.x * TILE; base < n; base += (u64)gridDim.x * TILE) {
+    for (u64 base = (u64)g.id * TILE; base < n; base += (u64)g.n * TILE) {
         for (u32 i = threadIdx.x; i < H; i += BLOCK) {
             hk[i] = kEmptyKey;
             ht[i] = 0u;
@@ -420,7 +421,7 @@ __device__ __forceinline__ void phase_mark(const BatchDev &b, const TablesDev &T
 template <int BLOCK, int IPT, int WB>
 __global__ void __launch_bounds__(BLOCK) k_mark(BatchDev b, TablesDev T, Scratch s, Counters *ctr) {
     pdl_begin();
-    phase_mark<BLOCK, IPT, WB>(b, T, s, ctr);
+    phase_mark<BLOCK, IPT, WB>(b, T, s, ctr, whole_grid());
 }
 
 // ============================================================================
@@ -440,10 +441,10 @@ __device__ __forceinline__ bool ids_dense(const Counters *ctr) {
 
 // Per contended cell: its address width (bit 63 of dcell marks an int64
 // cell), its value before the batch, and (priority rule) the min-writer slot.
-__device__ __forceinline__ void phase_dbase(const TablesDev &T, const Scratch &s, Counters *ctr, bool priority) {
+__device__ __forceinline__ void phase_dbase(const TablesDev &T, const Scratch &s, Counters *ctr, bool priority, const Grid g) {
     if (block_err(ctr)) return;
     const u64 M = ctr->M;
-    for (u64 m = (u64)blockIdx.x * blockDim.x + threadIdx.x; m < M; m += (u64)gridDim.x * blockDim.x) {
+    for (u64 m = (u64)g.id * blockDim.x + threadIdx.x; m < M; m += (u64)g.n * blockDim.x) {
         if (!LTP_IN_BOUNDS(ctr, m, s.cap_ops)) continue;
         const u64 cell = s.dcell[m];
         bool wide_c;
@@ -456,11 +457,11 @@ __device__ __forceinline__ void phase_dbase(const TablesDev &T, const Scratch &s
 
 __global__ void __launch_bounds__(256) k_dbase(TablesDev T, Scratch s, Counters *ctr, int priority) {
     pdl_begin();
-    phase_dbase(T, s, ctr, priority != 0);
+    phase_dbase(T, s, ctr, priority != 0, whole_grid());
 }
 
 template <int BLK, int WB>
-__device__ __forceinline__ void phase_ids(const TablesDev &T, const Scratch &s, Counters *ctr) {
+__device__ __forceinline__ void phase_ids(const TablesDev &T, const Scratch &s, Counters *ctr, const Grid g) {
     typedef typename Wd<WB>::T WT;
     constexpr u32 IPT = kIdsTile / BLK;
     if (block_err(ctr)) return;
@@ -471,11 +472,11 @@ __device__ __forceinline__ void phase_ids(const TablesDev &T, const Scratch &s, 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __shared__ u32 s_warp[BLK / 32];
     __shared__ u64 s_prefix;
-    if (blockIdx.x == 0 && threadIdx.x < T.n) {  // room for this batch's inserts?
+    if (g.id == 0 && threadIdx.x < T.n) {  // room for this batch's inserts?
         const u32 tb = threadIdx.x;
         if (T.rows_now[tb] + ctr->ins_total[tb] > T.t[tb].row_limit) set_err(ctr, LTP_E_CAPACITY);
     }
-    for (u32 tile = blockIdx.x; tile < tiles; tile += gridDim.x) {  // tiles wait for no other tile
+    for (u32 tile = g.id; tile < tiles; tile += g.n) {  // tiles wait for no other tile
         u32 wd[IPT];
         WT cw[IPT];
         u32 cnt = 0;
@@ -538,7 +539,7 @@ __device__ __forceinline__ void phase_ids(const TablesDev &T, const Scratch &s, 
 template <int WB>
 __global__ void __launch_bounds__(kIdsBlock) k_ids(TablesDev T, Scratch s, Counters *ctr) {
     pdl_begin();
-    phase_ids<kIdsBlock, WB>(T, s, ctr);
+    phase_ids<kIdsBlock, WB>(T, s, ctr, whole_grid());
 }
 
 // ============================================================================
@@ -701,7 +702,7 @@ __global__ void __launch_bounds__(BLOCK, 65536 / (BLOCK * (IPT <= 2 ? 40 : IPT <
 // predecessor tiles with relaxed loads, shared-memory staging so every
 // digit's run leaves as coalesced stores.
 template <int BLK>
-__device__ __forceinline__ void phase_sort_pass(const int P, const Scratch &s, Counters *ctr, u64 n_ops) {
+__device__ __forceinline__ void phase_sort_pass(const int P, const Scratch &s, Counters *ctr, u64 n_ops, const Grid g) {
     static_assert(BLK == 256, "one thread per radix digit");
     constexpr u32 SIPT = kSortTile / BLK;
     constexpr int WIN = 8;
@@ -715,7 +716,7 @@ __device__ __forceinline__ void phase_sort_pass(const int P, const Scratch &s, C
     u32 *status = s.st_sort[P & 1];
     if (P >= 1) {  // the previous pass is complete: recycle its look-back slots
         u32 *other = s.st_sort[(P + 1) & 1];
-        for (u64 j = (u64)blockIdx.x * BLK + threadIdx.x; j < (u64)tiles * 256; j += (u64)gridDim.x * BLK)
+        for (u64 j = (u64)g.id * BLK + threadIdx.x; j < (u64)tiles * 256; j += (u64)g.n * BLK)
             other[j] = 0;
     }
     constexpr int NW = BLK / 32;
@@ -862,7 +863,7 @@ __device__ __forceinline__ void phase_sort_pass(const int P, const Scratch &s, C
 template <int P>
 __global__ void __launch_bounds__(kSortBlock, 3) k_sort_pass(Scratch s, Counters *ctr, u64 n_ops) {
     pdl_begin();
-    phase_sort_pass<kSortBlock>(P, s, ctr, n_ops);
+    phase_sort_pass<kSortBlock>(P, s, ctr, n_ops, whole_grid());
 }
 
 // ============================================================================
@@ -1716,11 +1717,11 @@ __global__ void __launch_bounds__(kRowsBlock, MINB) k_rows(BatchDev b, TablesDev
 // ============================================================================
 template <int WB>
 __device__ __forceinline__ void phase_finish(const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
-                                             int rule) {
-    const u64 gsz = (u64)gridDim.x * blockDim.x, g0 = (u64)blockIdx.x * blockDim.x + threadIdx.x;
+                                             int rule, const Grid g) {
+    const u64 gsz = (u64)g.n * blockDim.x, g0 = (u64)g.id * blockDim.x + threadIdx.x;
     u32 any_ins = 0;
     for (u32 k = 0; k < T.n; k++) any_ins |= ctr->ins_total[k];
-    if (blockIdx.x == 0 && threadIdx.x < T.n && !ctr->err) T.rows_now[threadIdx.x] += ctr->ins_committed[threadIdx.x];
+    if (g.id == 0 && threadIdx.x < T.n && !ctr->err) T.rows_now[threadIdx.x] += ctr->ins_committed[threadIdx.x];
     if (any_ins) {
         const u64 t_ins = (b.n_ops + kInsTile - 1) / kInsTile;
         for (u64 j = g0; j < t_ins * LTP_MAX_TABLES; j += gsz) {
@@ -1774,7 +1775,7 @@ __device__ __forceinline__ void phase_finish(const BatchDev &b, const TablesDev 
 template <int WB>
 __global__ void __launch_bounds__(256) k_finish(BatchDev b, TablesDev T, Scratch s, Counters *ctr, int rule) {
     pdl_begin();
-    phase_finish<WB>(b, T, s, ctr, rule);
+    phase_finish<WB>(b, T, s, ctr, rule, whole_grid());
 }
 
 __global__ void k_stall(Counters *ctr, u32 ms) {
@@ -2077,77 +2078,144 @@ struct PersistArgs {
     Counters *one_snap;
 };
 
+// A grid of the blocks that happen to run: a block joins when it starts, the
+// first one closes the grid once every block of the launch has joined or,
+// beside other work on the GPU, none has for kJoinWaitNs.  Members are running
+// blocks, so they may wait for one another, which takes a cooperative launch
+// otherwise -- and that one waits until the whole grid has room at once (two
+// blocks of 128 registers a thread take every register of an SM: one sleeping
+// thread of another stream held a 100,000-op batch back until it ended, 280 ms
+// for 28 us).  False: not a member.
+constexpr u32 kJoinClosed = 1u << 31;
+constexpr u64 kJoinWaitNs = 20000ull;
+__device__ __forceinline__ bool join_grid(PartState *st, Counters *ctr, Counters *snap, Grid *g) {
+    __shared__ u32 s_id, s_n;
+    if (threadIdx.x == 0) {
+        const u32 id = atomicAdd(&st->joined, 1u);
+        u32 n = 0;
+        u64 t0 = gtimer();
+        if (id == 0) {
+            for (u32 seen = 1; seen < gridDim.x;) {
+                const u32 now = ld_acquire32(&st->joined);
+                if (now != seen) {
+                    seen = now;
+                    t0 = gtimer();
+                } else if (gtimer() - t0 > kJoinWaitNs) {
+                    break;
+                }
+            }
+            n = atomicOr(&st->joined, kJoinClosed);
+            st_release32(&st->members, n);
+        } else if (!(id & kJoinClosed)) {
+            while ((n = ld_acquire32(&st->members)) == 0u) {
+                if (gtimer() - t0 > kSpinLimitNs) {  // the other members' barriers give up on this
+                    set_err(ctr, LTP_E_TIMEOUT);
+                    set_err(snap, LTP_E_TIMEOUT);
+                    break;
+                }
+                __nanosleep(32);
+            }
+        }
+        s_id = id;
+        s_n = n;
+    }
+    __syncthreads();
+    g->id = s_id;
+    g->n = s_n;
+    return s_n != 0u;
+}
+
 constexpr int kPBlock = 256, kPIpt = 4;
 // dynamic shared memory of the persistent kernel: the larger of the mark
 // phase's hash (4 arrays of 2 x tile words) and the insert staging
 constexpr size_t kPersistSmem = 4ull * 2 * kPBlock * kPIpt * sizeof(u32) > kInsSmem
                                     ? 4ull * 2 * kPBlock * kPIpt * sizeof(u32) : (size_t)kInsSmem;
 
+// GATED: the bucket path's fallback (launch_fallback), else a cooperative launch.
+template <bool GATED>
 __global__ void __launch_bounds__(kPBlock, 2) k_persist(PersistArgs a) {
-    const u32 nb = gridDim.x;
-    if (a.gate) {
+    Grid joined = {};
+    if (GATED) {
         pdl_begin();
-        if (!*(volatile u32 *)&a.gate->skew) return;
+        if (!*(volatile u32 *)&a.gate->skew || !join_grid(a.gate, a.ctr, a.one_snap, &joined)) return;
     }
-    for (u32 j = 0; j < a.n_batches; j++) {
-        const BatchDev b = a.gate ? a.one : a.batches[j];
-        if (a.gate && b.payload_len) {  // the bucket path counted the inserts
+    auto g = [&]() { return GATED ? joined : whole_grid(); };
+    for (u32 j = 0; j < (GATED ? 1u : a.n_batches); j++) {
+        const BatchDev b = GATED ? a.one : a.batches[j];
+        if (GATED && b.payload_len) {  // the bucket path counted the inserts
             const u64 n = (b.n_ops + kInsTile - 1) / kInsTile * LTP_MAX_TABLES;
-            for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)nb * blockDim.x) a.s.ins_pre[i] = 0u;
+            for (u64 i = (u64)g().id * blockDim.x + threadIdx.x; i < n; i += (u64)g().n * blockDim.x) a.s.ins_pre[i] = 0u;
         }
-        if (blockIdx.x == 0) {  // fresh counters; a device error stays sticky for the run
+        if (!GATED && g().id == 0) {  // fresh counters; a device error stays sticky for the run
             const int keep = a.ctr->err;
             __syncthreads();
-            u32 *w = reinterpret_cast<u32 *>(a.ctr);
-            for (u32 i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) w[i] = 0u;
+            u32 *c = reinterpret_cast<u32 *>(a.ctr);
+            for (u32 i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) c[i] = 0;
             __syncthreads();
             if (threadIdx.x == 0) a.ctr->err = keep;
         }
-        for (u64 t = (u64)blockIdx.x * blockDim.x + threadIdx.x; t < b.n_txns; t += (u64)nb * blockDim.x) b.commit[t] = 1;
-        grid_sync(a.bar, nb, a.ctr);
+        for (u64 t = (u64)g().id * blockDim.x + threadIdx.x; t < b.n_txns; t += (u64)g().n * blockDim.x) b.commit[t] = 1;
+        grid_sync(a.bar, g().n, a.ctr);
         if (block_err(a.ctr)) break;
-        phase_mark<kPBlock, kPIpt, 32>(b, a.T, a.s, a.ctr);
-        grid_sync(a.bar, nb, a.ctr);
-        phase_ids<kPBlock, 32>(a.T, a.s, a.ctr);
-        grid_sync(a.bar, nb, a.ctr);
-        phase_dbase(a.T, a.s, a.ctr, a.rule == LTP_RULE_PRIORITY);
-        grid_sync(a.bar, nb, a.ctr);
-        if (a.rule != LTP_RULE_PRIORITY) {
+        phase_mark<kPBlock, kPIpt, 32>(b, a.T, a.s, a.ctr, g());
+        grid_sync(a.bar, g().n, a.ctr);
+        phase_ids<kPBlock, 32>(a.T, a.s, a.ctr, g());
+        grid_sync(a.bar, g().n, a.ctr);
+        phase_dbase(a.T, a.s, a.ctr, a.rule == LTP_RULE_PRIORITY, g());
+        grid_sync(a.bar, g().n, a.ctr);
+        if (GATED || a.rule != LTP_RULE_PRIORITY) {
             phase_classify<kPBlock, kPIpt, 32>(b, a.T, a.s, a.ctr);
-            grid_sync(a.bar, nb, a.ctr);
+            grid_sync(a.bar, g().n, a.ctr);
             // only the passes the contended ids need (M is the same for every
             // block after the barrier, so every block skips the same ones)
             const int passes = sort_passes_dev(*(volatile u32 *)&a.ctr->M);
             for (int P = 0; P < passes; P++) {
-                phase_sort_pass<kPBlock>(P, a.s, a.ctr, b.n_ops);
-                grid_sync(a.bar, nb, a.ctr);
+                phase_sort_pass<kPBlock>(P, a.s, a.ctr, b.n_ops, g());
+                grid_sync(a.bar, g().n, a.ctr);
             }
             if (a.T.any_wide && *(volatile u32 *)&a.ctr->wide_ops) phase_apply<kPBlock, u64>(b, a.T, a.s, a.ctr);
             else phase_apply<kPBlock, u32>(b, a.T, a.s, a.ctr);
         } else {
             phase_r1_minw<32, 1>(b, a.T, a.s, a.ctr);
-            grid_sync(a.bar, nb, a.ctr);
+            grid_sync(a.bar, g().n, a.ctr);
             phase_r1_abort<1>(b, a.s, a.ctr);
-            grid_sync(a.bar, nb, a.ctr);
+            grid_sync(a.bar, g().n, a.ctr);
             phase_r1_exec(b, a.T, a.s, a.ctr);
         }
-        grid_sync(a.bar, nb, a.ctr);
+        grid_sync(a.bar, g().n, a.ctr);
         if (b.payload_len) {  // a batch without payload has no valid insert
             phase_insert<kPBlock, false>(b, a.T, a.s, a.ctr);
-            grid_sync(a.bar, nb, a.ctr);
+            grid_sync(a.bar, g().n, a.ctr);
         }
-        phase_finish<32>(b, a.T, a.s, a.ctr, a.rule);
-        grid_sync(a.bar, nb, a.ctr);
-        if (blockIdx.x == 0) {
+        phase_finish<32>(b, a.T, a.s, a.ctr, a.rule, g());
+        if (GATED) break;
+        grid_sync(a.bar, g().n, a.ctr);
+        if (g().id == 0) {
             const u32 *src = reinterpret_cast<const u32 *>(a.ctr);
-            u32 *dst = reinterpret_cast<u32 *>(a.gate ? a.one_snap : a.snaps[j]);
+            u32 *dst = reinterpret_cast<u32 *>(a.snaps[j]);
             for (u32 i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) dst[i] = src[i];
         }
         if (block_err(a.ctr)) break;
-        grid_sync(a.bar, nb, a.ctr);
+        grid_sync(a.bar, g().n, a.ctr);
     }
-    if (a.gate && blockIdx.x == 0) {  // past the last barrier: every block has read the gate and the counters
-        for (u32 i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) reinterpret_cast<u32 *>(a.ctr)[i] = 0u;
+    if (GATED) {
+        // the last member to leave, on whichever way, is alone with the
+        // counters: it copies them and leaves them and the gate clean
+        __shared__ u32 s_last;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            s_last = atomicAdd(&a.gate->left, 1u) == g().n - 1u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!s_last) return;
+        volatile u32 *src = reinterpret_cast<volatile u32 *>(a.ctr);
+        u32 *dst = reinterpret_cast<u32 *>(a.one_snap);
+        for (u32 i = threadIdx.x; i < sizeof(Counters) / 4; i += blockDim.x) {
+            dst[i] = src[i];
+            src[i] = 0u;
+        }
         if (threadIdx.x == 0) a.gate->skew = 0u;
     }
 }
@@ -2158,9 +2226,9 @@ cudaError_t launch_persistent(cudaStream_t st, int num_sms, int rule, const Batc
     constexpr size_t smem = kPersistSmem;
     static int grid = 0, sms = 0;
     if (sms != num_sms) {
-        cudaError_t fe = cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t fe = cudaFuncSetAttribute(k_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (fe != cudaSuccess) return fe;
-        grid = occ_grid(k_persist, kPBlock, num_sms, smem);
+        grid = occ_grid(k_persist<false>, kPBlock, num_sms, smem);
         sms = num_sms;
     }
     (void)cudaGetLastError();
@@ -2177,18 +2245,23 @@ cudaError_t launch_persistent(cudaStream_t st, int num_sms, int rule, const Batc
     a.ctr = ctr;
     a.bar = bar;
     void *args[] = {&a};
-    return cudaLaunchCooperativeKernel((const void *)k_persist, dim3(grid), dim3(kPBlock), args, smem, st);
+    return cudaLaunchCooperativeKernel((const void *)k_persist<false>, dim3(grid), dim3(kPBlock), args, smem, st);
 }
 
+// By dependent launch: nearly always it only looks at the gate, and its launch
+// then hides behind the bucket kernel (six batches of 327,680 ops 311 -> 307
+// us, 65536 x 10 with snapshots 174 -> 170 us).
 cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *snap) {
     static int grid = 0, sms = 0;
     if (sms != L.num_sms) {
-        grid = persistent_grid(L.num_sms);
+        const cudaError_t e =
+            cudaFuncSetAttribute(k_persist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem);
+        if (e != cudaSuccess) return e;
+        grid = occ_grid(k_persist<true>, kPBlock, L.num_sms, kPersistSmem);
         sms = L.num_sms;
     }
     PersistArgs a;
     memset(&a, 0, sizeof(a));
-    a.n_batches = 1;
     a.rule = L.rule;
     a.T = T;
     a.s = s;
@@ -2197,28 +2270,13 @@ cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev 
     a.gate = s.pstate;
     a.one = b;
     a.one_snap = snap;
-    // Cooperative, and by dependent launch: nearly always it only looks at the
-    // gate, and its launch then hides behind the bucket kernel (six batches of
-    // 327,680 ops 311 -> 307 us, 65536 x 10 with snapshots 174 -> 170 us).
-    cudaLaunchConfig_t c = {};
-    c.gridDim = dim3(grid);
-    c.blockDim = dim3(kPBlock);
-    c.dynamicSmemBytes = kPersistSmem;
-    c.stream = L.stream;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = at;
-    c.numAttrs = 2;
-    return cudaLaunchKernelEx(&c, k_persist, a);
+    return launch_k(true, k_persist<true>, grid, kPBlock, kPersistSmem, L.stream, a);
 }
 
 int persistent_grid(int num_sms) {
     constexpr size_t smem = kPersistSmem;
-    cudaFuncSetAttribute(k_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return occ_grid(k_persist, kPBlock, num_sms, smem);
+    cudaFuncSetAttribute(k_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return occ_grid(k_persist<false>, kPBlock, num_sms, smem);
 }
 
 cudaError_t launch_reset_scratch(cudaStream_t st, const Scratch &s) {
