@@ -210,7 +210,8 @@ int ltp_batch_fetch64(ltp_ctx *ctx, ltp_batch *b, int64_t *vals, void *stream);
 /* Synchronises the stream, then fills stats (may be NULL) and reports any
  * device-side error of the batch. */
 int ltp_batch_finish(ltp_ctx *ctx, ltp_batch *b, ltp_stats *stats, void *stream);
-/* Convenience: fetch + finish. */
+/* Convenience: fetch + finish.  Several threads may take the results of
+ * different batches of a context at the same time. */
 int ltp_batch_results(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, ltp_stats *stats);
 /* The same with the full 64-bit values (ltp_batch_fetch64). */
 int ltp_batch_results64(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int64_t *vals, ltp_stats *stats);

@@ -832,7 +832,9 @@ int results_now(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, int6
     cudaStream_t st = ctx->stream;
     const uint64_t o_commit = (uint64_t)(b->commit - b->results), o_out = (uint64_t)((uint8_t *)b->out - b->results);
     const uint64_t nc = commit ? b->n_txns : 0, nv = vals ? b->n_ops * 4 : 0, nw = vals64 ? b->n_ops * 8 : 0;
-    uint8_t *h = ctx->h_stage;
+    // (another thread at it: straight into the caller's arrays)
+    std::unique_lock<std::mutex> staging(ctx->stage_mu, std::try_to_lock);
+    uint8_t *h = staging.owns_lock() ? ctx->h_stage : nullptr;
     if (!h || 2 * kOneCopyBytes + align256(nc) + align256(nv) + nw > kStageBytes) {
         int rc = ltp_batch_fetch(ctx, b, commit, vals, nullptr);
         if (!rc && vals64) rc = ltp_batch_fetch64(ctx, b, vals64, nullptr);
@@ -866,6 +868,7 @@ int results_now(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, int6
     if (nw) memcpy(vals64, h + used, nw);
     Counters c;
     memcpy(&c, h, kCounterHead);
+    staging.unlock();
     return finish_from(ctx, b, c, stats);
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -45,6 +46,7 @@ struct ltp_ctx {
     std::string last_error;
     Tuning tuning[64];
     uint32_t stall_ms_next = 0;
+    std::mutex stage_mu;         // held while h_stage is in use: results may be taken from several threads
     uint8_t *h_stage = nullptr;  // pinned staging of synchronous results (null: copied straight)
     bool dirty = false;  // scratch must be reset before the next batch
     // multi-batch execution: cached CUDA graph and persistent-kernel buffers
