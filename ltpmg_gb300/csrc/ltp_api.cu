@@ -56,6 +56,9 @@ cudaError_t dalloc(T **p, uint64_t count) {
 }
 
 // Pinned staging of a context, for results that come back synchronously.
+// Pinning and releasing it takes 105 + 165 us whatever its size, and a call
+// through it saves about 20 us: a context pins it when it is asked for results
+// a second time, so that one that is created for one batch does without.
 constexpr uint64_t kStageBytes = 1ull << 20;
 constexpr uint64_t kOneCopyBytes = 32u << 10;  // results that lie within this come back in one copy
 
@@ -87,36 +90,37 @@ void free_scratch_ops(Scratch &s) {
 }
 
 void free_scratch_words(Scratch &s) {
-    cudaFree(s.words);
-    cudaFree(s.cview);
-    cudaFree(s.word_epoch);
+    cudaFree(s.words);  // one allocation
     s.words = nullptr;
     s.cview = nullptr;
     s.word_epoch = nullptr;
 }
 
-// Sizes the bitmaps to the cell space and the per-op scratch to n_ops.
+// Sizes the bitmaps to the cell space and the per-op scratch to n_ops.  What
+// either holds starts over when one of them grows.
 int ensure_scratch(ltp_ctx *ctx, uint64_t n_ops) {
     Scratch &s = ctx->s;
     const uint64_t words = (ctx->total_cells + 31) / 32 + 1;
-    if (words > ctx->alloc_words) {
-        CK(cudaStreamSynchronize(ctx->stream));
+    const bool more_words = words > ctx->alloc_words, more_ops = n_ops > s.cap_ops;
+    if (!more_words && !more_ops) return LTP_OK;
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->dirty = true;  // until the end: an allocation may fail on the way
+    if (more_words) {
         free_scratch_words(s);
-        // one spare entry: the 64-cell layout of the same buffer rounds up
-        CK(dalloc(&s.words, words + 1));
-        CK(cudaMemset(s.words, 0, (words + 1) * sizeof(WordState)));
-        CK(dalloc(&s.cview, words + 1));  // 8 B per 32 cells; the 64-cell view takes 16 B per word
-        CK(cudaMemset(s.cview, 0, (words + 1) * sizeof(uint2)));
-        CK(dalloc(&s.word_epoch, words));
-        s.n_words = words;
-        CK(launch_reset_buckets(cudaStreamLegacy, s));  // the stamps start over
-        CK(cudaStreamSynchronize(cudaStreamLegacy));
+        ctx->alloc_words = 0;
+        // one spare entry: the 64-cell layout of the same buffer rounds up;
+        // the view takes 8 B per 32 cells, the 64-cell one 16 B per word
+        // (one allocation: each takes 35-80 us, and as long to free)
+        const uint64_t o_view = align256((words + 1) * sizeof(WordState));
+        const uint64_t o_epoch = o_view + align256((words + 1) * sizeof(uint2));
+        CK(cudaMalloc((void **)&s.words, o_epoch + words * 4));
+        s.cview = (uint2 *)((char *)s.words + o_view);
+        s.word_epoch = (u32 *)((char *)s.words + o_epoch);
         ctx->scratch_gen++;
         ctx->alloc_words = words;
     }
     s.n_words = words;
-    if (n_ops > s.cap_ops) {
-        CK(cudaStreamSynchronize(ctx->stream));
+    if (more_ops) {
         free_scratch_ops(s);
         uint64_t cap = 1024;
         while (cap < n_ops) cap <<= 1;
@@ -138,9 +142,10 @@ int ensure_scratch(ltp_ctx *ctx, uint64_t n_ops) {
         s.cap_ops = cap;
         s.cap_tiles = tiles;
         s.cap_sort_tiles = stiles;
-        CK(launch_reset_scratch(ctx->stream, s));
-        CK(cudaStreamSynchronize(ctx->stream));
     }
+    CK(launch_reset_scratch(ctx->stream, s));
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->dirty = false;
     return LTP_OK;
 }
 
@@ -201,23 +206,18 @@ int ltp_init(const ltp_config *cfg, ltp_ctx **out) {
     // (a limit of this process's context only)
     if (e == cudaSuccess) cudaDeviceSetLimit(cudaLimitMaxL2FetchGranularity, 32);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->ctr, sizeof(Counters));
-    if (e == cudaSuccess) e = cudaMemset(ctx->ctr, 0, sizeof(Counters));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->s.pctr, 2 * sizeof(PartCounters));
-    if (e == cudaSuccess) e = cudaMemset(ctx->s.pctr, 0, 2 * sizeof(PartCounters));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->s.fctr, sizeof(Counters));
-    if (e == cudaSuccess) e = cudaMemset(ctx->s.fctr, 0, sizeof(Counters));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->s.pstate, sizeof(PartState));
-    if (e == cudaSuccess) e = cudaMemset(ctx->s.pstate, 0, sizeof(PartState));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->rows_now, LTP_MAX_TABLES * sizeof(u64));
-    if (e == cudaSuccess) e = cudaMemset(ctx->rows_now, 0, LTP_MAX_TABLES * sizeof(u64));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&ctx->small, sizeof(SmallState));
+    if (e == cudaSuccess) e = cudaMemset(ctx->small, 0, sizeof(SmallState));
+    if (e == cudaSuccess) {
+        ctx->ctr = &ctx->small->ctr;
+        ctx->s.pctr = ctx->small->pctr;
+        ctx->s.fctr = &ctx->small->fctr;
+        ctx->s.pstate = &ctx->small->pstate;
+        ctx->rows_now = ctx->small->rows_now;
+    }
     if (e != cudaSuccess) {
         ltp_shutdown(ctx);
         return e == cudaErrorMemoryAllocation ? LTP_E_NOMEM : LTP_E_CUDA;
-    }
-    if (cudaMallocHost((void **)&ctx->h_stage, kStageBytes) != cudaSuccess) {  // without it, results are copied straight
-        (void)cudaGetLastError();
-        ctx->h_stage = nullptr;
     }
     if (cfg->reserve_ops) {
         int rc = ensure_scratch(ctx, cfg->reserve_ops);
@@ -237,11 +237,7 @@ int ltp_shutdown(ltp_ctx *ctx) {
     for (auto &t : ctx->tables) cudaFree(t.dev.data);
     free_scratch_ops(ctx->s);
     free_scratch_words(ctx->s);
-    cudaFree(ctx->ctr);
-    cudaFree(ctx->s.pctr);
-    cudaFree(ctx->s.fctr);
-    cudaFree(ctx->s.pstate);
-    cudaFree(ctx->rows_now);
+    cudaFree(ctx->small);
     if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
     if (ctx->p_exec) cudaGraphExecDestroy(ctx->p_exec);
     cudaFree(ctx->p_batches);
@@ -820,6 +816,15 @@ int finish_from(ltp_ctx *ctx, ltp_batch *b, const Counters &c, ltp_stats *stats)
     return LTP_OK;
 }
 
+// The context's pinned staging, from its second use on (its lock is held).
+uint8_t *stage_of(ltp_ctx *ctx) {
+    if (!ctx->h_stage && ctx->stage_uses++ == 1 && cudaMallocHost((void **)&ctx->h_stage, kStageBytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        ctx->h_stage = nullptr;
+    }
+    return ctx->h_stage;
+}
+
 // Results of an executed batch on the context's stream, synchronously: all of
 // a small batch's in as few copies as possible, through pinned memory, with
 // one wait (three copies to pageable memory wait one by one: 33 us of a
@@ -832,10 +837,11 @@ int results_now(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, int6
     cudaStream_t st = ctx->stream;
     const uint64_t o_commit = (uint64_t)(b->commit - b->results), o_out = (uint64_t)((uint8_t *)b->out - b->results);
     const uint64_t nc = commit ? b->n_txns : 0, nv = vals ? b->n_ops * 4 : 0, nw = vals64 ? b->n_ops * 8 : 0;
+    const bool fits = 2 * kOneCopyBytes + align256(nc) + align256(nv) + nw <= kStageBytes;
     // (another thread at it: straight into the caller's arrays)
     std::unique_lock<std::mutex> staging(ctx->stage_mu, std::try_to_lock);
-    uint8_t *h = staging.owns_lock() ? ctx->h_stage : nullptr;
-    if (!h || 2 * kOneCopyBytes + align256(nc) + align256(nv) + nw > kStageBytes) {
+    uint8_t *h = fits && staging.owns_lock() ? stage_of(ctx) : nullptr;
+    if (!h) {
         int rc = ltp_batch_fetch(ctx, b, commit, vals, nullptr);
         if (!rc && vals64) rc = ltp_batch_fetch64(ctx, b, vals64, nullptr);
         return rc ? rc : ltp_batch_finish(ctx, b, stats, nullptr);

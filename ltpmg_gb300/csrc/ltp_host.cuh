@@ -29,6 +29,15 @@ struct TableHost {
     char *col_ptr(uint32_t col, uint64_t row) const { return dev.data + col_off(dev, col) + row * width(col); }
 };
 
+// Device state of a context that does not grow, one allocation.
+struct SmallState {
+    alignas(256) Counters ctr;
+    alignas(256) ltp::PartCounters pctr[2];
+    alignas(256) Counters fctr;
+    alignas(256) ltp::PartState pstate;
+    alignas(256) u64 rows_now[LTP_MAX_TABLES];
+};
+
 struct ltp_ctx {
     int device = 0;
     int rule = LTP_RULE_ORDERED;
@@ -41,6 +50,7 @@ struct ltp_ctx {
     Scratch s;
     uint64_t alloc_words = 0;  // bitmap words currently allocated
     uint64_t scratch_gen = 0;  // counts scratch allocations: captured launches hold scratch pointers
+    SmallState *small = nullptr;
     Counters *ctr = nullptr;
     u64 *rows_now = nullptr;  // [LTP_MAX_TABLES] device row counts
     std::string last_error;
@@ -48,6 +58,7 @@ struct ltp_ctx {
     uint32_t stall_ms_next = 0;
     std::mutex stage_mu;         // held while h_stage is in use: results may be taken from several threads
     uint8_t *h_stage = nullptr;  // pinned staging of synchronous results (null: copied straight)
+    uint64_t stage_uses = 0;     // calls that found none
     bool dirty = false;  // scratch must be reset before the next batch
     // multi-batch execution: cached CUDA graph and persistent-kernel buffers
     std::vector<uint64_t> graph_key;

@@ -212,8 +212,6 @@ cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev 
 // Is (threads per block, ops per thread, conflict-word bits) a built tiling?
 bool tiling_supported(int block, int ipt, int word_bits);
 cudaError_t launch_reset_scratch(cudaStream_t st, const Scratch &s);
-// The bucket path's counters, state and stamps (part of the above).
-cudaError_t launch_reset_buckets(cudaStream_t st, const Scratch &s);
 cudaError_t launch_fill_seeded(cudaStream_t st, const TableDev &t, u64 seed);
 cudaError_t launch_expand_op_txn(cudaStream_t st, const u32 *txn_first, u64 n_txns, u32 *op_txn);
 // The same for a txn_first the host has not checked: a malformed one sets

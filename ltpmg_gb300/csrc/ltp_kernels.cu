@@ -2279,26 +2279,25 @@ int persistent_grid(int num_sms) {
     return occ_grid(k_persist<false>, kPBlock, num_sms, smem);
 }
 
+// All of it together: the bucket path's state says which of its counters the
+// next batch finds clean, and its stamps are compared with the words'.
 cudaError_t launch_reset_scratch(cudaStream_t st, const Scratch &s) {
     cudaMemsetAsync(s.words, 0, (s.n_words + 1) * sizeof(WordState), st);  // + the 64-cell layout's spare entry
     cudaMemsetAsync(s.cview, 0, (s.n_words + 1) * sizeof(uint2), st);
-    cudaMemsetAsync(s.st_sort[0], 0, s.cap_sort_tiles * 256 * 4, st);
-    cudaMemsetAsync(s.st_sort[1], 0, s.cap_sort_tiles * 256 * 4, st);
-    cudaMemsetAsync(s.st_cls, 0, s.cap_tiles * 8, st);
-    cudaMemsetAsync(s.st_apply, 0, s.cap_tiles * 8, st);
-    cudaMemsetAsync(s.st_ins, 0, s.cap_tiles * LTP_MAX_TABLES * 4, st);
-    if (s.ins_pre != s.st_ins) cudaMemsetAsync(s.ins_pre, 0, s.cap_tiles * LTP_MAX_TABLES * 4, st);
-    if (s.pctr) return launch_reset_buckets(st, s);
-    return cudaGetLastError();
-}
-
-// All of it together: the state says which counters the next batch finds
-// clean, and its stamps are compared with the words'.
-cudaError_t launch_reset_buckets(cudaStream_t st, const Scratch &s) {
-    cudaMemsetAsync(s.pctr, 0, 2 * sizeof(PartCounters), st);
-    cudaMemsetAsync(s.fctr, 0, sizeof(Counters), st);
-    cudaMemsetAsync(s.pstate, 0, sizeof(PartState), st);
-    cudaMemsetAsync(s.word_epoch, 0, s.n_words * 4, st);
+    if (s.cap_ops) {
+        cudaMemsetAsync(s.st_sort[0], 0, s.cap_sort_tiles * 256 * 4, st);
+        cudaMemsetAsync(s.st_sort[1], 0, s.cap_sort_tiles * 256 * 4, st);
+        cudaMemsetAsync(s.st_cls, 0, s.cap_tiles * 8, st);
+        cudaMemsetAsync(s.st_apply, 0, s.cap_tiles * 8, st);
+        cudaMemsetAsync(s.st_ins, 0, s.cap_tiles * LTP_MAX_TABLES * 4, st);
+        if (s.ins_pre != s.st_ins) cudaMemsetAsync(s.ins_pre, 0, s.cap_tiles * LTP_MAX_TABLES * 4, st);
+    }
+    if (s.pctr) {
+        cudaMemsetAsync(s.pctr, 0, 2 * sizeof(PartCounters), st);
+        cudaMemsetAsync(s.fctr, 0, sizeof(Counters), st);
+        cudaMemsetAsync(s.pstate, 0, sizeof(PartState), st);
+        cudaMemsetAsync(s.word_epoch, 0, s.n_words * 4, st);
+    }
     return cudaGetLastError();
 }
 

@@ -39,3 +39,17 @@ def test_results_of_two_batches_from_two_threads(lib, n_ops, wide):
         for t in threads:
             t.join()
         assert not failed and wrong == [0, 0]
+
+
+@pytest.mark.parametrize("n_ops", [700, 60000, 400000])  # one copy back, a copy per array, more than the staging holds
+def test_first_and_later_results_of_a_context_agree(lib, n_ops):
+    with G.Context(device=0) as ctx:
+        ctx.create_table(n_ops, 2)
+        ctx.fill_seeded(0, 3)
+        want = ctx.download(0)[0]
+        b = ctx.batch(n_ops, n_ops)
+        b.load(None, np.arange(n_ops, dtype=np.uint64), np.full(n_ops, G.opword(G.OP_ADD, 0, imm=7), np.uint32), ops_per_txn=1)
+        for k in range(4):
+            b.execute()
+            commit, vals, st = b.results()
+            assert commit.all() and st.committed == n_ops and np.array_equal(vals, want + np.int32(7 * (k + 1)))
