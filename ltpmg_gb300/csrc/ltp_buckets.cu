@@ -38,6 +38,7 @@
 #include <atomic>
 
 #include "ltp_device.cuh"
+#include "ltp_smem.h"
 #include "ltp_trace.h"
 
 namespace ltp {
@@ -1467,22 +1468,9 @@ u32 bits_for(u64 count) {  // bits that number `count` things, at least 1
     return b;
 }
 
-// Raises a kernel's shared-memory limit, once per device.
-template <typename K>
-cudaError_t allow_smem(K kernel, size_t bytes, std::atomic<u64> &done) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    const u64 bit = 1ull << (dev & 63);
-    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
-    return e;
-}
-
 template <class C>
 cudaError_t go_solo(const Launch &L, const BatchDev &b, const TablesDev &T, const BucketPlan &p) {
-    static std::atomic<u64> done{0};
+    static std::atomic<uint64_t> done{0};
     cudaError_t e = allow_smem(k_solo<C>, C::BYTES_SOLO, done);
     if (e == cudaSuccess) e = launch_k(L.pdl, k_solo<C>, 1, C::BLOCK, C::BYTES_SOLO, L.stream, b, T, p);
     return e;
@@ -1490,7 +1478,7 @@ cudaError_t go_solo(const Launch &L, const BatchDev &b, const TablesDev &T, cons
 
 template <class C>
 cudaError_t go_bucket(const Launch &L, const BatchDev &b, const TablesDev &T, const BucketPlan &p) {
-    static std::atomic<u64> done{0};
+    static std::atomic<uint64_t> done{0};
     cudaError_t e = allow_smem(k_bucket<C>, C::BYTES, done);
     const u32 grid = p.n_buckets + (b.payload_len ? 1u : 0u);
     if (e == cudaSuccess) e = launch_k(true, k_bucket<C>, grid, C::BLOCK, C::BYTES, L.stream, b, T, p);
@@ -1502,7 +1490,7 @@ cudaError_t go_bucket(const Launch &L, const BatchDev &b, const TablesDev &T, co
 // blocks would take shared memory while the bucket kernel runs, does not)
 template <int IPT>
 cudaError_t go_part(const Launch &L, const BatchDev &b, const TablesDev &T, const BucketPlan &p) {
-    static std::atomic<u64> done{0};
+    static std::atomic<uint64_t> done{0};
     cudaError_t e = allow_smem(k_part<IPT>, part_smem(kPartBlock * IPT, kMaxBuckets), done);
     if (e == cudaSuccess)
         e = launch_k(true, k_part<IPT>, p.n_tiles, kPartBlock, part_smem(p.tile, p.n_buckets), L.stream, b, T, p);

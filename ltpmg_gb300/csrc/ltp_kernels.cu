@@ -44,7 +44,10 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <atomic>
+
 #include "ltp_device.cuh"
+#include "ltp_smem.h"
 #include "ltp_trace.h"
 
 namespace ltp {
@@ -1850,10 +1853,9 @@ struct Front {
     static int g_mark, g_cls, sms;
     static constexpr size_t kMarkSmem = mark_smem_bytes<BLOCK, IPT, WB>();
     static void grids(int num_sms) {
+        static std::atomic<uint64_t> done{0};
+        if (allow_smem(k_mark<BLOCK, IPT, WB>, kMarkSmem, done) != cudaSuccess) return;  // the launch below then reports the error
         if (sms != num_sms) {
-            if (cudaFuncSetAttribute(k_mark<BLOCK, IPT, WB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kMarkSmem) != cudaSuccess)
-                return;  // the launch below then reports the error
             g_mark = occ_grid(k_mark<BLOCK, IPT, WB>, BLOCK, num_sms, kMarkSmem);
             g_cls = occ_grid(k_classify<BLOCK, IPT, WB>, BLOCK, num_sms);
             sms = num_sms;
@@ -1909,11 +1911,11 @@ static int capped(int grid, u64 upper) { return (int)((u64)grid < upper ? (u64)g
 template <int BLOCK, int MINB>
 static cudaError_t go_rows(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *ctr,
                            const PartState *ps) {
+    static std::atomic<uint64_t> done{0};
     static int grid = 0, sms = 0;
+    const cudaError_t e = allow_smem(k_rows<BLOCK, MINB>, kRowsSmem, done);
+    if (e != cudaSuccess) return e;
     if (sms != L.num_sms) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_rows<BLOCK, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowsSmem);
-        if (e != cudaSuccess) return e;
         grid = occ_grid(k_rows<BLOCK, MINB>, BLOCK, L.num_sms, kRowsSmem);
         sms = L.num_sms;
     }
@@ -1927,10 +1929,11 @@ cudaError_t launch_insert(const Launch &L, const BatchDev &b, const TablesDev &T
         // few rows per op: see k_rows
         return b.payload_len < b.n_ops / 4 ? go_rows<256, 3>(L, b, T, s, ctr, ps) : go_rows<512, 2>(L, b, T, s, ctr, ps);
     }
+    static std::atomic<uint64_t> done{0};
     static int gins = 0, sms = 0;
+    const cudaError_t e = allow_smem(k_insert, kInsSmemDesc, done);
+    if (e != cudaSuccess) return e;
     if (sms != L.num_sms) {
-        const cudaError_t e = cudaFuncSetAttribute(k_insert, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInsSmemDesc);
-        if (e != cudaSuccess) return e;
         gins = occ_grid(k_insert, kInsBlock, L.num_sms, kInsSmemDesc);
         sms = L.num_sms;
     }
@@ -2220,14 +2223,19 @@ __global__ void __launch_bounds__(kPBlock, 2) k_persist(PersistArgs a) {
     }
 }
 
+static cudaError_t allow_persist() {
+    static std::atomic<uint64_t> done{0};
+    return allow_smem(k_persist<false>, kPersistSmem, done);
+}
+
 cudaError_t launch_persistent(cudaStream_t st, int num_sms, int rule, const BatchDev *d_batches,
                               Counters *const *d_snaps, u32 n_batches, const TablesDev &T, const Scratch &s,
                               Counters *ctr, u32 *bar) {
     constexpr size_t smem = kPersistSmem;
     static int grid = 0, sms = 0;
+    cudaError_t fe = allow_persist();
+    if (fe != cudaSuccess) return fe;
     if (sms != num_sms) {
-        cudaError_t fe = cudaFuncSetAttribute(k_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (fe != cudaSuccess) return fe;
         grid = occ_grid(k_persist<false>, kPBlock, num_sms, smem);
         sms = num_sms;
     }
@@ -2252,11 +2260,11 @@ cudaError_t launch_persistent(cudaStream_t st, int num_sms, int rule, const Batc
 // then hides behind the bucket kernel (six batches of 327,680 ops 311 -> 307
 // us, 65536 x 10 with snapshots 174 -> 170 us).
 cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *snap) {
+    static std::atomic<uint64_t> done{0};
     static int grid = 0, sms = 0;
+    const cudaError_t e = allow_smem(k_persist<true>, kPersistSmem, done);
+    if (e != cudaSuccess) return e;
     if (sms != L.num_sms) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_persist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPersistSmem);
-        if (e != cudaSuccess) return e;
         grid = occ_grid(k_persist<true>, kPBlock, L.num_sms, kPersistSmem);
         sms = L.num_sms;
     }
@@ -2274,9 +2282,8 @@ cudaError_t launch_fallback(const Launch &L, const BatchDev &b, const TablesDev 
 }
 
 int persistent_grid(int num_sms) {
-    constexpr size_t smem = kPersistSmem;
-    cudaFuncSetAttribute(k_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return occ_grid(k_persist<false>, kPBlock, num_sms, smem);
+    (void)allow_persist();
+    return occ_grid(k_persist<false>, kPBlock, num_sms, kPersistSmem);
 }
 
 // All of it together: the bucket path's state says which of its counters the
