@@ -929,7 +929,7 @@ int ltp_set_tuning(ltp_ctx *ctx, uint32_t bucket, const ltp_tuning *t) {
     if (t->word_bits != 32 && t->word_bits != 64) return fail(ctx, LTP_E_BADARG, "word_bits must be 32 or 64");
     if (!tiling_supported((int)t->block, (int)t->ipt, (int)t->word_bits))
         return fail(ctx, LTP_E_BADARG, "64-cell conflict words need block x ipt <= 2048");
-    if (t->flags & ~LTP_TUNE_MARK_PRECHECK) return fail(ctx, LTP_E_BADARG, "unknown tuning flag");
+    if (t->flags & ~(LTP_TUNE_MARK_PRECHECK | LTP_TUNE_CONFLICT_WORDS)) return fail(ctx, LTP_E_BADARG, "unknown tuning flag");
     ctx->tuning[bucket] = Tuning{t->block, t->ipt, t->word_bits, t->flags};
     return LTP_OK;
 }

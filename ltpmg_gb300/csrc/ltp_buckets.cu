@@ -1506,6 +1506,7 @@ constexpr u32 kMaxLcBits = 28;                     // the slot word holds a cell
 bool plan_buckets(const Launch &L, const BatchDev &b, const TablesDev &T, const Scratch &s, Counters *snap, BucketPlan *p,
                   bool *solo) {
     if (L.rule == LTP_RULE_PRIORITY || L.stall || !s.pctr || T.n == 0 || b.n_ops == 0 || b.n_ops > kPartOps) return false;
+    if (L.tune.flags & LTP_TUNE_CONFLICT_WORDS) return false;
     const TableDev &lt = T.t[T.n - 1];
     const u64 cells = lt.cell_base + lt.row_limit * lt.n_cols;
     const u32 cb = bits_for(cells), n = (u32)b.n_ops;

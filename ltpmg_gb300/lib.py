@@ -96,6 +96,7 @@ class Tuning(ctypes.Structure):
 
 
 TUNE_MARK_PRECHECK = 1
+TUNE_CONFLICT_WORDS = 2
 
 
 _lib = None
