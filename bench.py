@@ -78,22 +78,34 @@ def mean_counters(stats):
     return {k: sum(s[k] for s in stats) / len(stats) for k in ("ops", "touched_words", "contended_cells", "contended_ops")}
 
 
-def stage_report(stats, extra):
+def by_buckets(n_ops, tiles):
+    """Does an ordered-rule batch go by buckets under these tunings (by size
+    bucket)?  64-cell words keep batches of more than 32,767 ops off them."""
+    import ltpmg_gb300 as G
+    from ltpmg_gb300 import autotune as AT
+
+    t = tiles.get(AT.bucket_of(n_ops), {})
+    if n_ops > BUCKET_OPS or t.get("flags", 0) & G.lib.TUNE_CONFLICT_WORDS:
+        return False
+    return t.get("word_bits", 32) == 32 or n_ops <= 32767
+
+
+def stage_report(stats, tiles, extra):
     """Average kernel times, algorithmic bytes per launch and mean counters
     of the batches of the path (conflict words or buckets) that takes more
     of the time; extra: further counters."""
     groups = {True: [], False: []}
     for s in stats:
-        groups[s["ops"] <= BUCKET_OPS].append(s)
-    by_buckets = max(groups, key=lambda k: sum(sum(s["ms_stage"].values()) for s in groups[k]))
-    g = groups[by_buckets]
+        groups[by_buckets(s["ops"], tiles)].append(s)
+    buckets = max(groups, key=lambda k: sum(sum(s["ms_stage"].values()) for s in groups[k]))
+    g = groups[buckets]
     mean = dict(mean_counters(g), **extra)
-    kernels = BUCKET_BYTES if by_buckets else {k: (k, f) for k, f in KERNEL_BYTES.items()}
+    kernels = BUCKET_BYTES if buckets else {k: (k, f) for k, f in KERNEL_BYTES.items()}
     avg = {k: sum(s["ms_stage"][stage] for s in g) / len(g) for k, (stage, _) in kernels.items()}
-    return by_buckets, avg, {k: f(mean) for k, (_, f) in kernels.items()}, mean
+    return buckets, avg, {k: f(mean) for k, (_, f) in kernels.items()}, mean
 
 
-def kernels_per_batch(n_ops, has_payload):
+def kernels_per_batch(n_ops, has_payload, tiles):
     """Kernels one batch launches under the ordered rule.  By buckets: split
     (not for one block's batch) and bucket, the insert kernel and the closing
     one with a payload, and from 32,768 ops on the fallback for skewed
@@ -101,7 +113,7 @@ def kernels_per_batch(n_ops, has_payload):
     classify, one radix pass per 8 bits of the largest possible contended id
     (n_ops - 1), apply, the insert prefix and insert (only with a payload),
     finish."""
-    if n_ops <= BUCKET_OPS:
+    if by_buckets(n_ops, tiles):
         return (1 if n_ops <= 2048 else 2) + (2 if has_payload else 0) + (1 if n_ops > 32767 else 0)
     passes = 1
     while passes < 4 and ((max(n_ops, 1) - 1) >> (8 * passes)) != 0:
@@ -536,29 +548,28 @@ def run_ours(args, config):
                          "achieved": alg / (step_ms / 1e3) / 1e9, "frac": alg / (step_ms / 1e3) / 1e9 / peak}}
     mean_stats = mean_counters(stats)
     if mode != G.MODE_PERSISTENT:
-        by_buckets, avg, kernel_bytes, path_stats = stage_report(stats, {"key_bytes": key_bytes})
+        buckets, avg, kernel_bytes, path_stats = stage_report(stats, tiles, {"key_bytes": key_bytes})
         dom = max(avg, key=avg.get)
         dom_bytes = kernel_bytes[dom]
         achieved = dom_bytes / (avg[dom] / 1e3) / 1e9
         traffic_b = measured_traffic(config, dom, path_stats)
         roof.update({"kernel": dom, "achieved": achieved, "frac": achieved / peak, "traffic": traffic_b,
                      "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": avg[dom], "kernel_ms": avg})
-        if not by_buckets:
+        if not buckets:
             roof["random_access"] = random_access_roof(G, local, sh, path_stats, avg, config)
     else:
         roof.update({"kernel": "k_persist (whole pipeline, one launch per step)", "achieved":
                      roof["pipeline"]["achieved"], "frac": roof["pipeline"]["frac"], "traffic": None,
                      "algorithmic_bytes_per_launch": alg, "avg_launch_ms": step_ms})
     launches = args.steps * (1 if mode == G.MODE_PERSISTENT else
-                             sum(kernels_per_batch(len(h[1]), False) for h in host))
+                             sum(kernels_per_batch(len(h[1]), False, tiles) for h in host))
     line = {"metric": METRIC, "value": value, "unit": "txn/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "int32", "data": "synthetic (seeded generator)",
             "config": {"workload": WORKLOAD_TEXT[config], "batches_per_step": nb, "txns_per_step": txns_per_step,
                        "rule": "ordered (ascending TID per cell, all commit)", "mode": mode_name,
                        "mode_ms": {str(k): v for k, v in mode_ms.items()},
-                       "tuning": {str(k): f"{v['block']}x{v['ipt']}" + ("w64" if v.get("word_bits") == 64 else "") + ("+precheck" if v.get("flags") else "")
-                                  for k, v in tiles.items()},
+                       "tuning": {str(k): v["name"] for k, v in tiles.items()},
                        "l2": "inputs larger than L2", "parallelism": f"replicas x{world}"},
             "gpu_launches": launches, "roofline": roof, "clocks": clk, "e2e": e2e,
             "contention": {"contended_ops_per_batch": mean_stats["contended_ops"],
@@ -578,19 +589,13 @@ def run_ours(args, config):
 def fixed_tiles(ctx, dev, spec):
     from ltpmg_gb300 import autotune as AT
 
-    import ltpmg_gb300 as G
-
-    # BLOCKxIPT[w64][+precheck], e.g. 512x4, 256x2w64+precheck
-    base, _, opt = spec.partition("+")
-    base, _, wb = base.partition("w")
-    blk, ipt = (int(x) for x in base.split("x"))
-    word_bits = int(wb) if wb else 32
-    flags = G.lib.TUNE_MARK_PRECHECK if opt == "precheck" else 0
+    # BLOCKxIPT[w64][+precheck][+words], e.g. 512x4, 256x2w64+precheck
+    blk, ipt, word_bits, flags = AT.parse_choice(spec)
     out = {}
     for b in dev:
         k = AT.bucket_of(b.n_ops)
         ctx.set_tuning(k, blk, ipt, word_bits=word_bits, flags=flags)
-        out[k] = {"block": blk, "ipt": ipt, "word_bits": word_bits, "flags": flags}
+        out[k] = {"name": spec, "block": blk, "ipt": ipt, "word_bits": word_bits, "flags": flags}
     return out
 
 
@@ -866,7 +871,7 @@ def run_payload(args, config):
     mean_stats = mean_counters(stats)
     if mode != G.MODE_PERSISTENT:
         _, avg, kernel_bytes, path_stats = stage_report(
-            stats, {"insert_bytes": sum(wl.insert_bytes(h) for h in host) / len(host), "key_bytes": 4})
+            stats, tiles, {"insert_bytes": sum(wl.insert_bytes(h) for h in host) / len(host), "key_bytes": 4})
         dom = max(avg, key=avg.get)
         dom_bytes = kernel_bytes[dom]
         achieved = dom_bytes / (avg[dom] / 1e3) / 1e9
@@ -878,7 +883,7 @@ def run_payload(args, config):
                      "achieved": roof["pipeline"]["achieved"], "frac": roof["pipeline"]["frac"], "traffic": None,
                      "algorithmic_bytes_per_launch": alg, "avg_launch_ms": step_ms})
     launches = args.steps * (1 if mode == G.MODE_PERSISTENT else
-                             sum(kernels_per_batch(len(h[1]), True) for h in host))
+                             sum(kernels_per_batch(len(h[1]), True, tiles) for h in host))
     rows = {wl.table_names()[t]: ctx.table_rows(tid) for t, tid in enumerate(ctx_tables)}
     line = {"metric": METRIC, "value": value, "unit": "txn/s", "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": step_ms, "higher_is_better": True,
@@ -886,8 +891,7 @@ def run_payload(args, config):
             "config": {"workload": WORKLOAD_TEXT[config], "batches_per_step": nb, "txns_per_step": txns_per_step,
                        "ops_per_step": ops_per_step, "rule": "ordered (ascending TID per cell, all commit)",
                        "mode": mode_name, "mode_ms": {str(k): v for k, v in mode_ms.items()},
-                       "tuning": {str(k): f"{v['block']}x{v['ipt']}" + ("w64" if v.get("word_bits") == 64 else "") + ("+precheck" if v.get("flags") else "")
-                                  for k, v in tiles.items()},
+                       "tuning": {str(k): v["name"] for k, v in tiles.items()},
                        "l2": "inputs larger than L2", "parallelism": f"replicas x{world}"},
             "gpu_launches": launches, "roofline": roof, "clocks": clk, "e2e": e2e,
             "contention": {"contended_ops_per_batch": mean_stats["contended_ops"],
@@ -1045,8 +1049,7 @@ def serving_measure(args, local, rank, point_s):
             if pf_ is not None:
                 bt.load_payload(pay_[int(pf_[0]):int(pf_[m])])
             ch = AT.tune_tiles(ctx, bt, reps=2)
-            chosen[ch["bucket"]] = f"{ch['block']}x{ch['ipt']}" + ("w64" if ch["word_bits"] == 64 else "") + \
-                ("+precheck" if ch["flags"] else "")
+            chosen[ch["bucket"]] = ch["name"]
             bt.finish()
             del bt
             truncate()
@@ -1256,7 +1259,7 @@ def main():
     ap.add_argument("--batches", type=int, default=0, help="resident batches (default: the config's)")
     ap.add_argument("--tuning-out", default="", help="write the autotuner's choices to this JSON file")
     ap.add_argument("--tiles", default="",
-                    help="fixed BLOCKxIPT[w64][+precheck] tiling instead of the autotuner's (e.g. 512x4, 256x2w64)")
+                    help="fixed BLOCKxIPT[w64][+precheck][+words] tiling instead of the autotuner's (e.g. 512x4, 256x2w64)")
     ap.add_argument("--no-e2e", action="store_true", help="skip the end-to-end pipeline pass")
     ap.add_argument("--loads", default="1,2,5,10,20,50", help="serving sweep: offered loads in M txn/s")
     ap.add_argument("--loadgen-threads", type=int, default=8, help="serving sweep: load-generator threads")

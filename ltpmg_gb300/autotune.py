@@ -5,8 +5,11 @@ tiling of the streaming kernels -- threads per block x ops per thread, the
 knobs that set how many ops a tile stages in shared memory -- then 64-cell
 conflict words (bitmap word granularity) for the fastest tilings, then the
 mark kernel's hot-word pre-check, on a representative batch with CUDA
-events, and keeps the fastest.  For a list of
-batches it also times the multi-batch execution modes (CUDA graph vs the
+events, and keeps the fastest.  Ordered-rule batches of up to 2^21 ops are
+executed by buckets of cells, whatever the tiling: there the candidates are
+the buckets and the conflict-word kernels in every tiling
+(TUNE_CONFLICT_WORDS), which are faster when one cell takes thousands of a
+batch's ops.  For a list of batches it also times the multi-batch execution modes (CUDA graph vs the
 persistent cooperative kernel) and keeps the faster one.  Choices persist as
 JSON and are applied with Context.set_tuning.
 
@@ -22,6 +25,7 @@ from . import lib as L
 
 BLOCKS = (128, 256, 512)
 IPTS = (1, 2, 4, 8)
+BUCKET_OPS = 2 << 20  # the largest ordered-rule batch that goes by buckets of cells
 
 
 def bucket_of(n_ops):
@@ -53,9 +57,17 @@ def _time_batch(ctx, batch, reps, copies=1):
     return ms[len(ms) // 2]
 
 
+def choice_name(block, ipt, word_bits=32, flags=0):
+    """Name of a tiling among the candidates (parse_choice is its inverse)."""
+    return (f"{block}x{ipt}" + ("w64" if word_bits == 64 else "") +
+            ("+precheck" if flags & L.TUNE_MARK_PRECHECK else "") + ("+words" if flags & L.TUNE_CONFLICT_WORDS else ""))
+
+
 def tune_tiles(ctx, batch, reps=3, blocks=BLOCKS, ipts=IPTS, copies=1):
     """Times every (block, ipt) on one loaded batch; sets and returns the best
-    for the batch's size bucket as {"block", "ipt", "ms", "candidates"}.
+    for the batch's size bucket as {"block", "ipt", "ms", "candidates"}.  A
+    batch that goes by buckets of cells is timed that way once ("buckets"),
+    then by conflict words in every tiling ("512x4+words").
     copies > 1 times graph-captured back-to-back executions (see _time_batch);
     a batch with insert payload is always timed one execution at a time, so
     that tuning appends as few rows as possible."""
@@ -65,29 +77,36 @@ def tune_tiles(ctx, batch, reps=3, blocks=BLOCKS, ipts=IPTS, copies=1):
     results = {}
     batch.execute()  # warm-up
     batch.finish()
+    by_buckets = getattr(ctx, "rule", None) == L.RULE_ORDERED and batch.n_ops <= BUCKET_OPS
+    words = L.TUNE_CONFLICT_WORDS if by_buckets else 0
+
+    def time_tiling(blk, ipt, word_bits=32, flags=0):
+        ctx.set_tuning(bucket, blk, ipt, word_bits=word_bits, flags=flags | words)
+        results[choice_name(blk, ipt, word_bits, flags | words)] = _time_batch(ctx, batch, reps, copies)
+
     for blk in blocks:
         for ipt in ipts:
-            ctx.set_tuning(bucket, blk, ipt)
-            results[f"{blk}x{ipt}"] = _time_batch(ctx, batch, reps, copies)
+            time_tiling(blk, ipt)
     # conflict-word granularity: 64-cell words for the three fastest tilings
     # that have them (tiles of at most 2048 ops)
+    n_w64 = 0
     for name in sorted(results, key=results.get)[:6]:
-        blk, ipt = (int(x) for x in name.split("x"))
-        if blk * ipt <= 2048 and len([k for k in results if k.endswith("w64")]) < 3:
-            ctx.set_tuning(bucket, blk, ipt, word_bits=64)
-            results[f"{name}w64"] = _time_batch(ctx, batch, reps, copies)
-    best = min(results, key=results.get)
-    base, _, wb = best.partition("w")
-    blk, ipt = (int(x) for x in base.split("x"))
-    word_bits = int(wb) if wb else 32
+        blk, ipt = parse_choice(name)[:2]
+        if blk * ipt <= 2048 and n_w64 < 3:
+            time_tiling(blk, ipt, 64)
+            n_w64 += 1
     # then, for the best tiling, the mark kernel's hot-word pre-check
-    ctx.set_tuning(bucket, blk, ipt, word_bits=word_bits, flags=L.TUNE_MARK_PRECHECK)
-    pre_ms = _time_batch(ctx, batch, reps, copies)
-    results[f"{best}+precheck"] = pre_ms
-    flags = L.TUNE_MARK_PRECHECK if pre_ms < results[best] else 0
+    blk, ipt, word_bits, _ = parse_choice(min(results, key=results.get))
+    time_tiling(blk, ipt, word_bits, L.TUNE_MARK_PRECHECK)
+    if by_buckets:
+        ctx.set_tuning(bucket, *parse_choice("buckets")[:2])
+        results["buckets"] = _time_batch(ctx, batch, reps, copies)
+    # (a tie goes to the one timed first among the tilings: without the pre-check)
+    best = min(results, key=results.get)
+    blk, ipt, word_bits, flags = parse_choice(best)
     ctx.set_tuning(bucket, blk, ipt, word_bits=word_bits, flags=flags)
-    return {"bucket": bucket, "block": blk, "ipt": ipt, "word_bits": word_bits, "flags": flags,
-            "ms": min(results[best], pre_ms), "candidates": results}
+    return {"bucket": bucket, "name": best, "block": blk, "ipt": ipt, "word_bits": word_bits, "flags": flags,
+            "ms": results[best], "candidates": results}
 
 
 def tune_mode(ctx, batches, reps=2, modes=(L.MODE_GRAPH, L.MODE_PERSISTENT)):
@@ -115,11 +134,16 @@ def tune_mode(ctx, batches, reps=2, modes=(L.MODE_GRAPH, L.MODE_PERSISTENT)):
 
 def parse_choice(name):
     """(block, ipt, word_bits, flags) of a candidate name such as 512x4,
-    512x2w64 or 512x4+precheck."""
-    base, _, opt = name.partition("+")
+    512x2w64, 512x4+precheck, 512x4+words or buckets."""
+    if name == "buckets":  # (no tiling matters there: the library's own)
+        name = "512x4"
+    base, *opts = name.split("+")
     base, _, wb = base.partition("w")
     blk, ipt = (int(x) for x in base.split("x"))
-    return blk, ipt, int(wb) if wb else 32, L.TUNE_MARK_PRECHECK if opt == "precheck" else 0
+    flags = 0
+    for opt in opts:
+        flags |= {"precheck": L.TUNE_MARK_PRECHECK, "words": L.TUNE_CONFLICT_WORDS}[opt]
+    return blk, ipt, int(wb) if wb else 32, flags
 
 
 def _time_list(ctx, batches, reps, mode=L.MODE_GRAPH):
@@ -155,12 +179,17 @@ def refine_pipeline(ctx, batches, choice, top=2, reps=2, mode=L.MODE_GRAPH):
     insert capacity."""
     bases = []
     for name in sorted(choice["candidates"], key=choice["candidates"].get):
-        base = name.partition("+")[0]
+        base = name.replace("+precheck", "")
         if base not in bases:
             bases.append(base)
         if len(bases) == top:
             break
-    ranked = [b + sfx for b in bases for sfx in ("", "+precheck")]
+    ranked = []
+    for b in bases:
+        ranked.append(b)
+        if b != "buckets":
+            blk, ipt, wb, flags = parse_choice(b)
+            ranked.append(choice_name(blk, ipt, wb, flags | L.TUNE_MARK_PRECHECK))
     timed = {}
     for name in ranked:
         blk, ipt, wb, flags = parse_choice(name)
@@ -170,7 +199,7 @@ def refine_pipeline(ctx, batches, choice, top=2, reps=2, mode=L.MODE_GRAPH):
     blk, ipt, wb, flags = parse_choice(best)
     ctx.set_tuning(choice["bucket"], blk, ipt, word_bits=wb, flags=flags)
     out = dict(choice)
-    out.update({"block": blk, "ipt": ipt, "word_bits": wb, "flags": flags, "pipeline_ms": timed})
+    out.update({"name": best, "block": blk, "ipt": ipt, "word_bits": wb, "flags": flags, "pipeline_ms": timed})
     return out
 
 
