@@ -1456,7 +1456,11 @@ __global__ void __launch_bounds__(1024) k_end(BatchDev b, TablesDev T, BucketPla
     const u64 n = (b.n_ops + kInsTile - 1) / kInsTile * LTP_MAX_TABLES;
     for (u64 j = tid; j < n; j += blockDim.x) p.ins_pre[j] = 0u;
     __syncthreads();
-    if (tid == 0) p.state->full = 0u;
+    if (tid == 0) {
+        p.state->full = 0u;
+        // noted since the snapshot was taken (a bounds check of the row kernel)
+        if (c->err && !p.snap->err) p.snap->err = c->err;
+    }
 }
 
 // ============================================================================
