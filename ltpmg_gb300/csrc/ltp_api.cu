@@ -841,6 +841,10 @@ int results_now(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, int6
     // (another thread at it: straight into the caller's arrays)
     std::unique_lock<std::mutex> staging(ctx->stage_mu, std::try_to_lock);
     uint8_t *h = fits && staging.owns_lock() ? stage_of(ctx) : nullptr;
+    // without a staging, small results still come back in one copy
+    const bool one_copy = o_out + nv <= kOneCopyBytes;
+    alignas(16) uint8_t local[kOneCopyBytes];
+    if (!h && one_copy && !nw) h = local;
     if (!h) {
         int rc = ltp_batch_fetch(ctx, b, commit, vals, nullptr);
         if (!rc && vals64) rc = ltp_batch_fetch64(ctx, b, vals64, nullptr);
@@ -848,7 +852,7 @@ int results_now(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, int6
     }
     const uint8_t *hc, *hv;
     uint64_t used;
-    if (o_out + nv <= kOneCopyBytes) {  // counters, commit flags and values as they lie
+    if (one_copy) {  // counters, commit flags and values as they lie
         used = nv ? o_out + nv : o_commit + nc;
         CK(cudaMemcpyAsync(h, b->results, used, cudaMemcpyDeviceToHost, st));
         hc = h + o_commit;
@@ -874,7 +878,7 @@ int results_now(ltp_ctx *ctx, ltp_batch *b, uint8_t *commit, int32_t *vals, int6
     if (nw) memcpy(vals64, h + used, nw);
     Counters c;
     memcpy(&c, h, kCounterHead);
-    staging.unlock();
+    if (staging.owns_lock()) staging.unlock();
     return finish_from(ctx, b, c, stats);
 }
 
