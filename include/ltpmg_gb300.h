@@ -492,7 +492,7 @@ typedef struct {
  * by buckets of cells, where block, ipt and LTP_TUNE_MARK_PRECHECK have no
  * effect, and word_bits = 64 keeps batches of more than 32,767 ops on the
  * conflict words.  This flag keeps every batch of the size bucket there: the
- * faster way where a single cell takes more than about 8,000 of a batch's ops
+ * faster way where a single cell takes more than about 6,000 of a batch's ops
  * and some write it (e.g. 655,360 reads and read-modify-writes under Zipf 0.99
  * on one column: 163 us by buckets, 114 us by conflict words). */
 #define LTP_TUNE_CONFLICT_WORDS 2u

@@ -25,7 +25,9 @@ from . import lib as L
 
 BLOCKS = (128, 256, 512)
 IPTS = (1, 2, 4, 8)
-BUCKET_OPS = 2 << 20  # the largest ordered-rule batch that goes by buckets of cells
+# the largest ordered-rule batch, and the most cells of a context, that go by
+# buckets of cells
+BUCKET_OPS, BUCKET_CELLS = 2 << 20, 1 << 32
 
 
 def bucket_of(n_ops):
@@ -77,7 +79,8 @@ def tune_tiles(ctx, batch, reps=3, blocks=BLOCKS, ipts=IPTS, copies=1):
     results = {}
     batch.execute()  # warm-up
     batch.finish()
-    by_buckets = getattr(ctx, "rule", None) == L.RULE_ORDERED and batch.n_ops <= BUCKET_OPS
+    by_buckets = (getattr(ctx, "rule", None) == L.RULE_ORDERED and batch.n_ops <= BUCKET_OPS and
+                  getattr(ctx, "cells", 0) <= BUCKET_CELLS)
     words = L.TUNE_CONFLICT_WORDS if by_buckets else 0
 
     def time_tiling(blk, ipt, word_bits=32, flags=0):

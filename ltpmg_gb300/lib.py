@@ -369,6 +369,7 @@ class Context:
         self.h = h
         self.rule = rule
         self.tables = []
+        self.cells = 0  # cell numbers lie below this
 
     def check(self, rc):
         if rc != LTP_OK:
@@ -406,6 +407,7 @@ class Context:
         self.check(self.L.ltp_table_create_cap(self.h, ctypes.byref(Schema(cols, 0, mask)), rows, cap,
                                                ctypes.byref(tid)))
         self.tables.append((rows, cols, mask))
+        self.cells = (self.cells + 31) // 32 * 32 + cap * cols  # (a table starts with a conflict word)
         return tid.value
 
     def truncate(self, table, rows):

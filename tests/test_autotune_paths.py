@@ -56,8 +56,10 @@ def test_conflict_words_are_kept_when_faster(monkeypatch):
     assert ctx.tuning[20] == (256, 2, 32, PRE | WORDS) == AT.parse_choice(ch["name"])
 
 
-@pytest.mark.parametrize("rule,n_ops", [(L.RULE_PRIORITY, 1 << 20), (L.RULE_ORDERED, (2 << 20) + 1)])
-def test_batches_that_cannot_go_by_buckets(monkeypatch, rule, n_ops):
+@pytest.mark.parametrize("rule,n_ops,cells", [(L.RULE_PRIORITY, 1 << 20, 0), (L.RULE_ORDERED, (2 << 20) + 1, 0),
+                                              (L.RULE_ORDERED, 1 << 20, (1 << 32) + 1)])
+def test_batches_that_cannot_go_by_buckets(monkeypatch, rule, n_ops, cells):
+    monkeypatch.setattr(FakeCtx, "cells", cells, raising=False)
     ctx, ch = tune(monkeypatch, rule, n_ops, words_cost)
     assert ch["name"] == "256x2+precheck" and ch["flags"] == PRE
     assert not any(c[3] & WORDS for c in ctx.calls) and "buckets" not in ch["candidates"]
@@ -100,4 +102,5 @@ def test_tuned_path_of_a_real_batch(lib, hot):
         b = ctx.batch(n, n)
         b.load(None, cells.astype(np.uint32), opw, ops_per_txn=1)
         ch = AT.tune_tiles(ctx, b, reps=5, copies=4)
+        assert ctx.cells == space
         assert (ch["name"] != "buckets") == hot == bool(ctx.get_tuning(ch["bucket"])[3] & WORDS)
