@@ -80,7 +80,8 @@ def mean_counters(stats):
 
 def by_buckets(n_ops, tiles):
     """Does an ordered-rule batch go by buckets under these tunings (by size
-    bucket)?  64-cell words keep batches of more than 32,767 ops off them."""
+    bucket; contexts of at most 2^32 cells)?  64-cell words keep batches of
+    more than 32,767 ops off them."""
     import ltpmg_gb300 as G
     from ltpmg_gb300 import autotune as AT
 

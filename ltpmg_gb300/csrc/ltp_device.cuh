@@ -333,8 +333,9 @@ __device__ __forceinline__ u32 op_tid(const BatchDev &b, u64 i) {
 
 // Launches a batch kernel, with programmatic stream serialization when `pdl`
 // (see pdl_begin): it may start while its predecessor on the stream drains.
-// Stream launches use it; captured graphs do not (their launches already
-// follow each other closely, and measured no faster with it).
+// The caller chooses: stream launches use it always; inside captured graphs
+// the split and bucket kernels and the fallback do, the others in batches of
+// fewer than 2^18 ops (see launch_execute and go_part).
 template <typename... KP, typename... A>
 static cudaError_t launch_k(bool pdl, void (*kernel)(KP...), unsigned grid, unsigned block, size_t smem,
                             cudaStream_t st, A... args) {
